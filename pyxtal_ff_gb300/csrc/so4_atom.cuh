@@ -1,4 +1,4 @@
-// so4_atom.cuh -- per-centre-atom phases shared by the plain and adjoint kernels.
+// so4_atom.cuh -- U_tot of one centre per CTA (twol 0 and 1) and the small tables.
 // Each function is called by all threads of a CTA of NW warps and ends with
 // __syncthreads().
 #pragma once
@@ -52,81 +52,6 @@ __device__ void block_utot(const SmallTables &st, const T *rootpq, int a, const 
         Uh[e] = cscale(s, (T)st.unorm[l]);
     }
     __syncthreads();
-}
-
-// Full (l+1)^2 layers from the half layout by the inversion symmetry (SO4.py:908-925).
-template <typename T, int NW>
-__device__ void block_expand(const SmallTables &st, const cx<T> *Uh, int nu, cx<T> *Uf) {
-    const int ldim = st.twol + 1;
-    for (int f = threadIdx.x; f < nu; f += NW * 32) {
-        const int l = level_of(st.u_block, ldim, f);
-        const int off = f - st.u_block[l];
-        const int mb = off / (l + 1), ma = off - mb * (l + 1);
-        cx<T> v;
-        if (2 * mb <= l) {
-            v = Uh[st.h_block[l] + mb * (l + 1) + ma];
-        } else {
-            v = cconj(Uh[st.h_block[l] + (l - mb) * (l + 1) + (l - ma)]);
-            if ((mb + ma) & 1) {
-                v.re = -v.re;
-                v.im = -v.im;
-            }
-        }
-        Uf[f] = v;
-    }
-    __syncthreads();
-}
-
-// One Z entry (compute_zi, SO4.py:1020-1068).
-template <typename T>
-__device__ __forceinline__ cx<T> z_entry(const ZEnt &ze, const T *cg, const cx<T> *Uf) {
-    cx<T> zz = mk<T>(T(0), T(0));
-    int u1 = ze.u1 + ze.ma1min, u2 = ze.u2 + ze.ma2max, icgb = ze.cgb;
-    for (int ib = 0; ib < ze.nb; ++ib) {
-        cx<T> s = mk<T>(T(0), T(0));
-        int icga = ze.cga;
-        for (int ia = 0; ia < ze.na; ++ia) {
-            cfma(s, cscale(Uf[u1 + ia], cg[icga]), Uf[u2 - ia]);
-            icga += ze.l2;
-        }
-        zz = cadd(zz, cscale(s, cg[icgb]));
-        u1 += ze.l1 + 1;
-        u2 -= ze.l2 + 1;
-        icgb += ze.l2;
-    }
-    return zz;
-}
-
-template <typename T, int NW>
-__device__ void block_z(const ZEnt *zent, int nz, const T *cg, const cx<T> *Uf, cx<T> *Z) {
-    for (int q = threadIdx.x; q < nz; q += NW * 32) Z[q] = z_entry<T>(zent[q], cg, Uf);
-    __syncthreads();
-}
-
-// The Z entries of a list (e.g. only the blocks B reads), each to its own slot.
-template <typename T, int NW>
-__device__ void block_z_list(const ZEnt *list, int n, const T *cg, const cx<T> *Uf, cx<T> *Z) {
-    for (int q = threadIdx.x; q < n; q += NW * 32) {
-        const ZEnt ze = list[q];
-        Z[ze.jz] = z_entry<T>(ze, cg, Uf);
-    }
-    __syncthreads();
-}
-
-// B_k = 2 Re sum' conj(U_l) Z(l1,l2,l) (compute_bi, SO4.py:1071-1111).
-template <typename T, int NW, typename TO>
-__device__ void block_b(const BEnt *bent, int nB, const cx<T> *Uh, const cx<T> *Z, TO *x) {
-    for (int k = threadIdx.x; k < nB; k += NW * 32) {
-        const BEnt be = bent[k];
-        const int lam = be.lam[0], cnt = be.cnt[0];
-        T s = T(0);
-        for (int e = 0; e < cnt; ++e) {
-            T v = redot(Uh[be.h[0] + e], Z[be.z[0] + e]);
-            if ((lam % 2 == 0) && e == cnt - 1) v *= T(0.5);
-            s += v;
-        }
-        x[k] = (TO)(T(2) * s);
-    }
 }
 
 inline void fill_small_tables(const so4_tables *t, SmallTables &st) {

@@ -53,19 +53,6 @@ template <typename T>
 __device__ __forceinline__ T redot(cx<T> a, cx<T> b) { return a.re * b.re + a.im * b.im; }
 
 // ------------------------------------------------------------------ tables
-// One Z entry (SO4.py:1344-1395 idxz row) with its CG offset and the full-layout
-// offsets of the first U_l1 / U_l2 elements it reads.
-struct ZEnt {
-    int na, nb;          // inner / outer trip counts
-    int ma1min, ma2max;  // first column of U_l1, U_l2
-    int cga, cgb;        // CG offsets of the first inner / outer coefficient
-    int u1, u2;          // full offsets of U_l1[mb1min][0], U_l2[mb2max][0]
-    int l1, l2;          // row strides - 1
-    int jh;              // half offset of (l, mb, ma)
-    int blk;             // Z block index
-    int jz;              // index of this entry in the full Z list
-};
-
 // One bispectrum component k = (l1, l2, l), l >= l1 >= l2 (SO4.py:1314-1327),
 // with the three Z blocks its derivative reads (SO4.py:1113-1227).
 struct BEnt {
@@ -98,11 +85,8 @@ struct so4_tables {
     std::vector<int> h_block;  // ldim + 1
     std::vector<double> unorm_l;  // per level
     // device copies
-    double *d_cg64 = nullptr;
     float *d_cg32 = nullptr;
-    double *d_rootpq64 = nullptr;  // ldim x ldim
     float *d_rootpq32 = nullptr;
-    ZEnt *d_z = nullptr;
     BEnt *d_b = nullptr;
     ZBlk *d_blk = nullptr;
     // per Z block, packed for the window kernels' coefficient loop: the components of its
@@ -118,15 +102,33 @@ struct so4_tables {
     // it is finished (F the row scale of the scaled recursion, so4_tables.cu)
     int4 *d_hmap = nullptr;
     float *d_yscale = nullptr;  // n_half: the row-scale F of each half entry (so4_tables.cu)
-    double *d_yscale64 = nullptr;  // the same in FP64 (the plain path's scaled derivative pass)
-    // The plain path's dB/dr sections: every distinct Z block they read, contracted once per
-    // image by one lane of a warp, {first Z entry, half offset, entry count, level}, listed
-    // lane by lane (lane l owns [psec_ptr[l], psec_ptr[l + 1])) with the lanes' entry counts
-    // balanced; ksec[3 k + s]: the list position of component k's section s.
-    int4 *d_psec = nullptr;
-    int *d_psec_ptr = nullptr;  // 33
-    int *d_ksec = nullptr;      // 3 nB
-    int n_psec = 0;
+    // Plain path (so4_plain.cu).  Its arrays carry U in the scaled form V = U / F and Z as
+    // F Z (F the row scale), each Z block cut to its dB/dr section, blocks ordered by level.
+    //   pz_unit   Z work units, three int4 each, most expensive first: {full offsets of the
+    //             first U_l1 | U_l2 << 16, inner | outer trips << 8 | levels << 16, ca offset,
+    //             cb offset}, {row stride l1 + 1 | l2 + 1 << 16, coefficient pitch, output of
+    //             level 0, 1}, {output of level 2, 3, 0, 0}
+    //   pz_ca/cb  the Clebsch-Gordan factors of the inner and the outer sum, scaled
+    //   p_vent    n_half: the two entries of the level below that a U entry is made of
+    //   p_lam     per level {entries of a section, first block, blocks, first entry in p_sent}
+    //   p_blk     per block {component, first Z value, entries, level}; p_fac its factor
+    //             times u_norm
+    //   p_kblk    per component {up to three blocks, their number}
+    //   p_zent    per Z value: block | row exponent << 16
+    //   p_wpos, p_wfac  the same values component by component, component k owning entries
+    //             [p_wk[k], p_wk[k + 1]): what the FP32 kernel forms the generators' W of
+    //   p_sent    section entries of all levels: ma | centre of a middle row << 8 | exponent << 16
+    int4 *d_pz_unit = nullptr, *d_p_vent = nullptr, *d_p_lam = nullptr, *d_p_blk = nullptr, *d_p_kblk = nullptr;
+    double *d_pz_ca = nullptr, *d_pz_cb = nullptr;
+    float *d_pz_ca32 = nullptr, *d_pz_cb32 = nullptr;
+    double *d_p_fac = nullptr;
+    int *d_p_sent = nullptr;
+    int *d_p_bblk = nullptr;  // n_b: the block a component's B contracts
+    int *d_p_zent = nullptr, *d_p_wk = nullptr;
+    int4 *d_p_wpos = nullptr;
+    float4 *d_p_wfac = nullptr;
+    std::vector<int> p_wk;
+    int n_pz_unit = 0, n_pblk = 0, n_pz = 0;
     // B partial slots of the window kernels: one per (window unit, B block), component k
     // owning slots [bpos[k], bpos[k + 1]) in row order
     int *d_bpos = nullptr;  // nB + 1
@@ -150,6 +152,9 @@ struct so4_tables {
     int n_jmax = 0;  // the most slots one component owns
     int n_wsub = 0;  // window sub-segments
 };
+
+// Levels per Z unit of the plain path (so4_plain.cu).
+constexpr int PZ_G = 4;
 
 // Window Z contractions: most entries per unit, and the zero rows kept before
 // and after the U tiles in shared memory (a window may reach ZW_KMAX - 1 entries
@@ -408,102 +413,6 @@ template <typename T>
 __device__ __forceinline__ void cmsub(cx<T> &acc, const cx<T> &a, const cx<T> &b) {
     acc.re = fma(-a.re, b.re, fma(a.im, b.im, acc.re));
     acc.im = fma(-a.re, b.im, fma(-a.im, b.re, acc.im));
-}
-
-// warp_uarray in the scaled form V_l[mb][ma] = U_l[mb][ma] / F, F = sqrt(C(l, mb) / C(l, ma))
-// (C binomial; the row-scale table of so4_tables.cu).  The recursion's coefficients
-// rootpq[l-ma][l-mb] and rootpq[ma][l-mb] cancel against the scale:
-//   V_l[mb][ma] = conj(a) V_{l-1}[mb][ma] - conj(b) V_{l-1}[mb][ma-1],
-// and the chain-start mirror and the middle-row symmetry keep their form, because
-// C(l, ma) = C(l, l - ma).  So U = F V, and a contraction Re sum conj(dU) Z equals
-// Re sum conj(dV) (F Z): callers pre-scale Z by F instead of unscaling every row.
-// 56 FMAs per entry with DERIV against about 92 operations in warp_uarray.
-template <typename T, bool DERIV>
-__device__ void warp_vrows(const SmallTables &st, const CK<T> &ck, cx<T> *H, cx<T> *dH, int n_half, int lane) {
-    const int ldim = st.twol + 1;
-    if (lane == 0) {
-        H[0] = mk<T>(T(1), T(0));
-        if (DERIV) {
-            dH[0] = mk<T>(T(0), T(0));
-            dH[n_half] = mk<T>(T(0), T(0));
-            dH[2 * n_half] = mk<T>(T(0), T(0));
-        }
-    }
-    __syncwarp();
-    for (int l = 1; l < ldim; ++l) {
-        const int ncol = l + 1;
-        const int n = (l / 2 + 1) * ncol;
-        cx<T> *Hl = H + st.h_block[l];
-        const cx<T> *Hp = H + st.h_block[l - 1];
-        for (int e = lane; e < n; e += 32) {
-            const int mb = e / ncol;
-            const int ma = e - mb * ncol;
-            cx<T> v = mk<T>(T(0), T(0));
-            cx<T> dv[3];
-            if (DERIV) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) dv[c] = mk<T>(T(0), T(0));
-            }
-            if (ma > 0) {
-                const cx<T> P = prev_row(Hp, l, mb, ma - 1);
-                cmsub(v, ck.cb, P);
-                if (DERIV) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const cx<T> dP = prev_row(dH + c * n_half + st.h_block[l - 1], l, mb, ma - 1);
-                        cmsub(dv[c], ck.cdb[c], P);
-                        cmsub(dv[c], ck.cb, dP);
-                    }
-                }
-            }
-            if (ma < l) {
-                const cx<T> P = prev_row(Hp, l, mb, ma);
-                cmac(v, ck.ca, P);
-                if (DERIV) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        const cx<T> dP = prev_row(dH + c * n_half + st.h_block[l - 1], l, mb, ma);
-                        cmac(dv[c], ck.cda[c], P);
-                        cmac(dv[c], ck.ca, dP);
-                    }
-                }
-            }
-            Hl[e] = v;
-            if (DERIV) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) dH[c * n_half + st.h_block[l] + e] = dv[c];
-            }
-        }
-        __syncwarp();
-        if ((l & 1) == 0) {
-            // middle row mb = l/2: centre -> conj, upper half -> mirror of lower half
-            const int mid = (l / 2) * ncol;
-            const int h = l / 2;
-            for (int ma = h + lane; ma <= l; ma += 32) {
-                const int src = (ma == h) ? ma : (l - ma);
-                const bool neg = ((h + ma) & 1) != 0;
-                cx<T> v = cconj(Hl[mid + src]);
-                if (neg && ma != h) {
-                    v.re = -v.re;
-                    v.im = -v.im;
-                }
-                Hl[mid + ma] = v;
-                if (DERIV) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        cx<T> *dHl = dH + c * n_half + st.h_block[l];
-                        cx<T> dv = cconj(dHl[mid + src]);
-                        if (neg && ma != h) {
-                            dv.re = -dv.re;
-                            dv.im = -dv.im;
-                        }
-                        dHl[mid + ma] = dv;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
 }
 
 // Number of half-layout entries one dB/dr section of level lam sums over

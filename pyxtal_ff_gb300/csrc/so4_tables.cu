@@ -81,11 +81,8 @@ int upload(T **dst, const std::vector<T> &src) {
 }
 
 void free_device(so4_tables *t) {
-    cudaFree(t->d_cg64);
     cudaFree(t->d_cg32);
-    cudaFree(t->d_rootpq64);
     cudaFree(t->d_rootpq32);
-    cudaFree(t->d_z);
     cudaFree(t->d_b);
     cudaFree(t->d_blk);
     cudaFree(t->d_blk_rk);
@@ -95,10 +92,22 @@ void free_device(so4_tables *t) {
     cudaFree(t->d_hfull);
     cudaFree(t->d_hmap);
     cudaFree(t->d_yscale);
-    cudaFree(t->d_yscale64);
-    cudaFree(t->d_psec);
-    cudaFree(t->d_psec_ptr);
-    cudaFree(t->d_ksec);
+    cudaFree(t->d_pz_unit);
+    cudaFree(t->d_p_vent);
+    cudaFree(t->d_p_lam);
+    cudaFree(t->d_p_blk);
+    cudaFree(t->d_pz_ca);
+    cudaFree(t->d_pz_cb);
+    cudaFree(t->d_pz_ca32);
+    cudaFree(t->d_pz_cb32);
+    cudaFree(t->d_p_fac);
+    cudaFree(t->d_p_sent);
+    cudaFree(t->d_p_bblk);
+    cudaFree(t->d_p_kblk);
+    cudaFree(t->d_p_zent);
+    cudaFree(t->d_p_wpos);
+    cudaFree(t->d_p_wfac);
+    cudaFree(t->d_p_wk);
     cudaFree(t->d_bpos);
     cudaFree(t->d_wunit_y);
     cudaFree(t->d_wseg_y);
@@ -261,9 +270,8 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
                 }
     t->n_b = (int)t->idxb.size() / 3;
 
-    // idxz and idxz_block (SO4.py:1329-1395), plus the device entry list
+    // idxz and idxz_block (SO4.py:1329-1395)
     t->idxz_block.assign(ld * ld * ld, 0);
-    std::vector<ZEnt> zent;
     std::vector<ZBlk> blks;
     n = 0;
     for (int l1 = 0; l1 < ld; ++l1)
@@ -290,22 +298,6 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
                         q[8] = std::min(l1, (2 * mb - l + l2 + l1) / 2) - q[6] + 1;
                         q[9] = t->idxu_block[l] + (l + 1) * mb + ma;
                         for (int c = 0; c < 10; ++c) t->idxz.push_back(q[c]);
-                        ZEnt z;
-                        const int cgbase = t->idxcg_block[b3(ld, l1, l2, l)];
-                        z.na = q[5];
-                        z.nb = q[8];
-                        z.ma1min = q[3];
-                        z.ma2max = q[4];
-                        z.cga = cgbase + q[3] * (l2 + 1) + q[4];
-                        z.cgb = cgbase + q[6] * (l2 + 1) + q[7];
-                        z.u1 = t->idxu_block[l1] + (l1 + 1) * q[6];
-                        z.u2 = t->idxu_block[l2] + (l2 + 1) * q[7];
-                        z.l1 = l1;
-                        z.l2 = l2;
-                        z.jh = t->h_block[l] + (l + 1) * mb + ma;
-                        z.blk = (int)blks.size();
-                        z.jz = n;
-                        zent.push_back(z);
                         n++;
                     }
                 bk.n = n - bk.z0;
@@ -346,45 +338,196 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
                 }
         }
     }
-    // The plain path's dB/dr: the three sections of every component read Z blocks that
-    // several components share (165 sections over 125 distinct blocks at lmax 4), and the
-    // components' section sizes differ several-fold.  So each distinct block is contracted
-    // once per image, the blocks dealt to the 32 lanes of a warp largest first, each to the
-    // lane with the fewest entries so far (ties: the lower lane), and listed lane by lane.
-    std::vector<int4> usec;  // {first Z entry, half offset, entry count, level}
-    std::vector<int> ksec_u(3 * (size_t)t->n_b);
-    for (int k = 0; k < t->n_b; ++k)
-        for (int s = 0; s < 3; ++s) {
-            int u = 0;
-            while (u < (int)usec.size() && usec[u].x != bent[k].z[s]) ++u;
-            if (u == (int)usec.size()) usec.push_back(make_int4(bent[k].z[s], bent[k].h[s], bent[k].cnt[s], bent[k].lam[s]));
-            ksec_u[3 * k + s] = u;
-        }
-    std::vector<int> order(usec.size());
-    for (size_t u = 0; u < usec.size(); ++u) order[u] = (int)u;
-    std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return usec[p].z > usec[q].z; });
-    std::vector<int> lane_of(usec.size()), load(32, 0);
-    for (int u : order) {
-        int best = 0;
-        for (int l = 1; l < 32; ++l)
-            if (load[l] < load[best]) best = l;
-        lane_of[u] = best;
-        load[best] += usec[u].z;
-    }
-    std::vector<int4> psec;
-    std::vector<int> psec_ptr(33, 0), pos_of(usec.size());
-    for (int l = 0; l < 32; ++l) {
-        psec_ptr[l] = (int)psec.size();
-        for (int u : order)
-            if (lane_of[u] == l) {
-                pos_of[u] = (int)psec.size();
-                psec.push_back(usec[u]);
+    // The plain path's tables (so4_common.cuh).  F(l, mb, ma) = f(l, mb) / f(l, ma),
+    // f(l, m) = sqrt(C(l, m)): with U = F V and Z' = F Z every scale is a product of one factor
+    // per index, and the Z sums take V and give Z' with the factors inside the two tables:
+    //   Z'(mb, ma) = sum_{mb1} cb sum_{ma1} ca V_l1[mb1][ma1] V_l2[mb2][ma2].
+    auto binom = [](int l, int m) {
+        double c = 1.0;
+        for (int i = 1; i <= m; ++i) c = c * (double)(l - m + i) / (double)i;
+        return c;
+    };
+    auto f_of = [&](int l, int m) { return std::sqrt(binom(l, m)); };
+    // the power of two nearest to f(l, mb): V and Z' as integers are scaled per row by it and
+    // its inverse, so that V's rows use the same range
+    auto row_exp = [&](int l, int mb) { return (int)std::lround(std::log2(f_of(l, mb))); };
+    int prc = SO4_OK;
+    std::vector<int> pblk_of(t->n_blk, -1), p_zof, p_bblk(t->n_b), p_sent, p_zent;
+    std::vector<int4> p_blk, p_lam(ld), pz_unit, p_vent(nh), p_kblk(t->n_b, make_int4(0, 0, 0, 0));
+    std::vector<double> p_fac, pz_ca, pz_cb;
+    int pz = 0;
+    for (int lam = 0; lam < ld; ++lam) {
+        const int E = section_count(lam), first = (int)p_blk.size();
+        for (int bi = 0; bi < t->n_blk; ++bi) {
+            const ZBlk &bk = blks[bi];
+            if (bk.l != lam || bk.nrole == 0) continue;
+            // every role of a block belongs to one component, the one whose indices are the
+            // block's (largest first); equal indices give the block two or three roles there
+            double f = 0.0;
+            for (int r = 0; r < bk.nrole; ++r) {
+                if (bk.role_k[r] != bk.role_k[0]) prc = SO4_ERR_UNSUPPORTED;
+                f += bk.role_f[r] * t->unorm_l[lam];
             }
+            int4 &kb = p_kblk[bk.role_k[0]];
+            (kb.w == 0 ? kb.x : (kb.w == 1 ? kb.y : kb.z)) = (int)p_blk.size();
+            kb.w++;
+            pblk_of[bi] = (int)p_blk.size();
+            p_blk.push_back(make_int4(bk.role_k[0], pz, E, lam));
+            p_fac.push_back(f);
+            for (int e = 0; e < E; ++e) p_zent.push_back(pblk_of[bi] | (row_exp(lam, e / (lam + 1)) << 16));
+            p_zof.push_back(pz);
+            pz += E;
+        }
+        p_lam[lam] = make_int4(E, first, (int)p_blk.size() - first, (int)p_sent.size());
+        for (int e = 0; e < E; ++e) {
+            const int ma = e % (lam + 1), mb = e / (lam + 1);
+            p_sent.push_back(ma | ((2 * mb == lam && 2 * ma == lam) ? 1 << 8 : 0) | (row_exp(lam, mb) << 16));
+        }
     }
-    psec_ptr[32] = (int)psec.size();
-    std::vector<int> ksec(3 * (size_t)t->n_b);
-    for (size_t i = 0; i < ksec.size(); ++i) ksec[i] = pos_of[ksec_u[i]];
-    t->n_psec = (int)psec.size();
+    p_zof.push_back(pz);
+    t->n_pblk = (int)p_blk.size();
+    t->n_pz = pz;
+    for (int k = 0; k < t->n_b; ++k)
+        for (int bi = 0; bi < t->n_blk; ++bi)
+            if (blks[bi].z0 == bent[k].z[0]) p_bblk[k] = pblk_of[bi];
+    // FP32: W0..W3 of a block's entry are (w.x Z', -i w.y Z', w.z Z'[m+1] - w.w Z'[m-1],
+    // -i (w.z Z'[m+1] + w.w Z'[m-1])), with the block's factor and, at the centre of a middle
+    // row, the half weight inside; entries listed component by component
+    std::vector<int4> p_wpos;
+    std::vector<float4> p_wfac;
+    std::vector<int> p_wk(t->n_b + 1, 0);
+    for (int k = 0; k < t->n_b; ++k) {
+        const int bs[3] = {p_kblk[k].x, p_kblk[k].y, p_kblk[k].z};
+        for (int i = 0; i < p_kblk[k].w; ++i) {
+            const int4 b = p_blk[bs[i]];
+            for (int e = 0; e < b.z; ++e) {
+                const int ma = e % (b.w + 1), mb = e / (b.w + 1);
+                const bool ctr = 2 * mb == b.w && 2 * ma == b.w;
+                const double f = p_fac[bs[i]] * (ctr ? 0.5 : 1.0);
+                // positions of Z', Z'[m+1], Z'[m-1] (past a row's end: Z' itself, weight 0), and
+                // whether Z'[m+1] is the mirror -conj(Z'[m-1])
+                p_wpos.push_back(make_int4(b.y + e, b.y + e + (ctr ? (ma > 0 ? -1 : 0) : (ma < b.w ? 1 : 0)),
+                                           b.y + e - (ma > 0 ? 1 : 0), ctr ? 1 : 0));
+                p_wfac.push_back(make_float4((float)f, (float)(f * (b.w - 2 * ma)), (float)(f * (b.w - ma)), (float)(f * ma)));
+            }
+        }
+        p_wk[k + 1] = (int)p_wpos.size();
+    }
+    // U entry (l, mb, ma) = conj(a) P[ma] - conj(b) P[ma - 1], P row mb of level l - 1, or its
+    // mirror (-1)^(..) conj of row l - 1 - mb: {index of P[ma], of P[ma - 1] (-1: none),
+    // 1 conjugate | 2 negate P[ma] | 4 negate P[ma - 1], 1 middle-row centre | 2 ma = mb | l << 8 |
+    // row exponent << 16}
+    for (int l = 0; l < ld; ++l)
+        for (int mb = 0; 2 * mb <= l; ++mb)
+            for (int ma = 0; ma <= l; ++ma) {
+                int4 e = make_int4(-1, -1, 0, ((2 * mb == l && 2 * ma == l) ? 1 : 0) | (ma == mb ? 2 : 0) | (l << 8) | (row_exp(l, mb) << 16));
+                const int L = l - 1;
+                if (l > 0 && 2 * mb <= L) {
+                    if (ma < l) e.x = t->h_block[L] + mb * l + ma;
+                    if (ma > 0) e.y = t->h_block[L] + mb * l + ma - 1;
+                } else if (l > 0) {
+                    const int row = t->h_block[L] + (L - mb) * l;
+                    e.z = 1;
+                    if (ma < l) {
+                        e.x = row + (L - ma);
+                        e.z |= ((mb + ma) & 1) ? 2 : 0;
+                    }
+                    if (ma > 0) {
+                        e.y = row + (L - (ma - 1));
+                        e.z |= ((mb + ma - 1) & 1) ? 4 : 0;
+                    }
+                }
+                p_vent[t->h_block[l] + mb * (l + 1) + ma] = e;
+            }
+    // Z units: one (l1, l2, S, s), S = mb1 + mb2 and s = ma1 + ma2, for up to PZ_G of the levels
+    // whose section has that entry; the products V_l1 V_l2 are shared by the unit's levels
+    struct PUnit {
+        int n;
+        long cost;
+        int4 q[3];
+    };
+    std::vector<PUnit> pun;
+    for (int l1 = 0; l1 < ld; ++l1)
+        for (int l2 = 0; l2 <= l1; ++l2) {
+            const int L = l1 + l2;
+            std::vector<int> lams, bis;
+            for (int bi = 0; bi < t->n_blk; ++bi)
+                if (blks[bi].l1 == l1 && blks[bi].l2 == l2 && pblk_of[bi] >= 0) {
+                    lams.push_back(blks[bi].l);
+                    bis.push_back(pblk_of[bi]);
+                }
+            const int np = (int)lams.size();
+            if (!np) continue;
+            // With a, b, c = (l1 + l2 - l) / 2, (l1 - l2 + l) / 2, (-l1 + l2 + l) / 2 Racah's sum is
+            // CG(m1, m2) = N Delta sqrt((l + 1) m1! (l1 - m1)! m2! (l2 - m2)! m! (l - m)!) / (a! b! c!),
+            // N = sum_z (-1)^z C(a, z) C(b, l1 - m1 - z) C(c, m2 - z) an integer, and the factors f
+            // take the square roots away: the outer coefficients are the integers N, the inner
+            // ones kappa N / (C(l1, m1) C(l2, m2) C(l, m)),
+            // kappa = (l + 1) l1! l2! l! / (a! b! c! ((l1 + l2 + l) / 2 + 1)!).
+            auto nsum = [&](int lam, int m1, int m2) {
+                const int na = (L - lam) / 2, nb = (l1 - l2 + lam) / 2, nc = (l2 - l1 + lam) / 2;
+                double sum = 0.0;  // exact: far below 2^53
+                for (int z = 0; z <= std::min(na, std::min(l1 - m1, m2)); ++z)
+                    if (l1 - m1 - z <= nb && m2 - z <= nc)
+                        sum += ((z & 1) ? -1.0 : 1.0) * binom(na, z) * binom(nb, l1 - m1 - z) * binom(nc, m2 - z);
+                return sum;
+            };
+            auto kappa = [&](int lam) {  // one rounding each for numerator, denominator and quotient
+                unsigned __int128 num = lam + 1, den = 1;
+                for (int f : {l1, l2, lam})
+                    for (int i = 2; i <= f; ++i) num *= (unsigned)i;
+                for (int f : {(L - lam) / 2, (l1 - l2 + lam) / 2, (l2 - l1 + lam) / 2, (L + lam) / 2 + 1})
+                    for (int i = 2; i <= f; ++i) den *= (unsigned)i;
+                return (double)num / (double)den;
+            };
+            // coefficient rows [m1 - lo][level], one block per value of s (inner) and S (outer);
+            // with l1 = l2 the outer pairs (mb1, mb2) and (mb2, mb1) give the same sums, so only
+            // mb1 <= mb2 is walked, twice its weight where they differ
+            std::vector<int> ca_at(L + 1), cb_at(L + 1);
+            for (int s = 0; s <= L; ++s) {
+                ca_at[s] = (int)pz_ca.size();
+                cb_at[s] = (int)pz_cb.size();
+                for (int m1 = std::max(0, s - l2); m1 <= std::min(l1, s); ++m1)
+                    for (int q = 0; q < np; ++q) {
+                        const int m = s - (L - lams[q]) / 2, m2 = s - m1;
+                        const bool ok = m >= 0 && m <= lams[q];
+                        const double g = ok ? nsum(lams[q], m1, m2) : 0.0;
+                        const double c = binom(l1, m1) * binom(l2, m2) * (ok ? binom(lams[q], m) : 1.0);
+                        pz_ca.push_back(kappa(lams[q]) * g / c);
+                        pz_cb.push_back(g * ((l1 == l2 && 2 * m1 != s) ? 2.0 : 1.0));
+                    }
+            }
+            for (int S = 0; 2 * S <= L; ++S)
+                for (int s = 0; s <= L; ++s) {
+                    if (2 * S == L && 2 * s > L) continue;  // past the centre of every middle row
+                    std::vector<int> val;
+                    for (int q = 0; q < np; ++q)
+                        if (lams[q] >= std::abs(2 * s - L) && lams[q] >= L - 2 * S) val.push_back(q);
+                    const int lo = std::max(0, s - l2), na = std::min(l1, s) - lo + 1;
+                    const int Lo = std::max(0, S - l2), Hi = (l1 == l2) ? S / 2 : std::min(l1, S), nb = Hi - Lo + 1;
+                    for (size_t g = 0; g < val.size(); g += PZ_G) {
+                        PUnit u;
+                        u.n = (int)std::min<size_t>(PZ_G, val.size() - g);
+                        u.cost = (long)nb * (na * (4 + 2 * u.n) + 2 * u.n);
+                        const int u1 = t->idxu_block[l1] + Lo * (l1 + 1) + lo;
+                        const int u2 = t->idxu_block[l2] + (S - Lo) * (l2 + 1) + (s - lo);
+                        int out[PZ_G] = {0};
+                        for (int j = 0; j < u.n; ++j) {
+                            const int q = val[g + j], lam = lams[q], d = (L - lam) / 2;
+                            out[j] = p_zof[bis[q]] + (S - d) * (lam + 1) + (s - d);
+                        }
+                        u.q[0] = make_int4(u1 | (u2 << 16), na | (nb << 8) | (u.n << 16), ca_at[s] + val[g],
+                                           cb_at[S] + val[g]);
+                        u.q[1] = make_int4((l1 + 1) | ((l2 + 1) << 16), np, out[0], out[1]);
+                        u.q[2] = make_int4(out[2], out[3], 0, 0);
+                        pun.push_back(u);
+                    }
+                }
+        }
+    std::stable_sort(pun.begin(), pun.end(), [](const PUnit &p, const PUnit &q) { return p.cost > q.cost; });
+    for (const PUnit &u : pun) pz_unit.insert(pz_unit.end(), u.q, u.q + 3);
+    t->n_pz_unit = (int)pz_unit.size() / 3;
+    const std::vector<float> pz_ca32(pz_ca.begin(), pz_ca.end()), pz_cb32(pz_cb.begin(), pz_cb.end());
 
     // blocks grouped by their third index (the level of Y they feed)
     std::vector<int> yptr(ld + 1, 0), ylist;
@@ -395,13 +538,9 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     }
     yptr[ld] = (int)ylist.size();
 
-    std::vector<double> rp64(ld * ld, 0.0);
     std::vector<float> rp32(ld * ld, 0.f);
     for (int p = 1; p < ld; ++p)
-        for (int q = 1; q < ld; ++q) {
-            rp64[p * ld + q] = std::sqrt((double)p / (double)q);
-            rp32[p * ld + q] = (float)rp64[p * ld + q];
-        }
+        for (int q = 1; q < ld; ++q) rp32[p * ld + q] = (float)std::sqrt((double)p / (double)q);
     std::vector<float> cg32(t->cglist.begin(), t->cglist.end());
     // B component of each block (blocks with l >= l1)
     std::vector<int> blk_k(t->n_blk, -1);
@@ -673,14 +812,8 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     // symmetry keep their form.  hmap: per half entry {slot | row << 8 | diagonal << 15,
     // bits of u_norm F, bits of u_norm, 0}; yscale: F, by which the window kernels scale Y so
     // that the reverse sweep contracts V with it.
-    auto binom = [](int n, int k) {
-        double c = 1.0;
-        for (int i = 1; i <= k; ++i) c = c * (double)(n - k + i) / (double)i;
-        return c;
-    };
     std::vector<int4> hmap;
     std::vector<float> yscale;
-    std::vector<double> yscale64;
     for (int l = 0; l < ld; ++l) {
         const float un = (float)t->unorm_l[l];
         for (int mb = 0; 2 * mb <= l; ++mb)
@@ -692,13 +825,11 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
                 std::memcpy(&b_un, &un, sizeof b_un);
                 hmap.push_back(make_int4((l * (l + 1) / 2 + ma) | (mb << 8) | ((ma == mb ? 1 : 0) << 15), b_unf, b_un, 0));
                 yscale.push_back((float)F);
-                yscale64.push_back(F);
             }
     }
     if (!rc) rc = upload(&t->d_hfull, hfull);
     if (!rc) rc = upload(&t->d_hmap, hmap);
     if (!rc) rc = upload(&t->d_yscale, yscale);
-    if (!rc) rc = upload(&t->d_yscale64, yscale64);
     if (!rc) rc = upload(&t->d_bpos, bpos);
     if (!rc) rc = upload(&t->d_wunit_y, wunit_y);
     if (!rc) rc = upload(&t->d_wseg_y, wseg_y);
@@ -711,15 +842,27 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     if (!rc) rc = upload(&t->d_jbase, jbase);
     if (!rc) rc = upload(&t->d_jfac, jfac);
     if (!rc) rc = upload(&t->d_wca, wca);
-    if (!rc) rc = upload(&t->d_cg64, t->cglist);
     if (!rc) rc = upload(&t->d_cg32, cg32);
-    if (!rc) rc = upload(&t->d_rootpq64, rp64);
     if (!rc) rc = upload(&t->d_rootpq32, rp32);
-    if (!rc) rc = upload(&t->d_z, zent);
     if (!rc) rc = upload(&t->d_b, bent);
-    if (!rc) rc = upload(&t->d_psec, psec);
-    if (!rc) rc = upload(&t->d_psec_ptr, psec_ptr);
-    if (!rc) rc = upload(&t->d_ksec, ksec);
+    if (!rc) rc = upload(&t->d_pz_unit, pz_unit);
+    if (!rc) rc = upload(&t->d_p_vent, p_vent);
+    if (!rc) rc = upload(&t->d_p_lam, p_lam);
+    if (!rc) rc = upload(&t->d_p_blk, p_blk);
+    if (!rc) rc = upload(&t->d_pz_ca, pz_ca);
+    if (!rc) rc = upload(&t->d_pz_cb, pz_cb);
+    if (!rc) rc = upload(&t->d_pz_ca32, pz_ca32);
+    if (!rc) rc = upload(&t->d_pz_cb32, pz_cb32);
+    if (!rc) rc = upload(&t->d_p_fac, p_fac);
+    if (!rc) rc = upload(&t->d_p_sent, p_sent);
+    if (!rc) rc = upload(&t->d_p_bblk, p_bblk);
+    if (!rc) rc = upload(&t->d_p_kblk, p_kblk);
+    if (!rc) rc = upload(&t->d_p_zent, p_zent);
+    if (!rc) rc = upload(&t->d_p_wpos, p_wpos);
+    if (!rc) rc = upload(&t->d_p_wfac, p_wfac);
+    if (!rc) rc = upload(&t->d_p_wk, p_wk);
+    t->p_wk = p_wk;
+    if (!rc) rc = prc;
     if (!rc) rc = upload(&t->d_blk, blks);
     if (!rc) {
         std::vector<int4> rk(t->n_blk);
