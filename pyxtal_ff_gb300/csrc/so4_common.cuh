@@ -113,12 +113,12 @@ struct so4_tables {
     //   p_lam     per level {entries of a section, first block, blocks, first entry in p_sent}
     //   p_blk     per block {component, first Z value, entries, level}; p_fac its factor
     //             times u_norm
-    //   p_kblk    per component {up to three blocks, their number}
     //   p_zent    per Z value: block | row exponent << 16
-    //   p_wpos, p_wfac  the same values component by component, component k owning entries
-    //             [p_wk[k], p_wk[k + 1]): what the FP32 kernel forms the generators' W of
+    //   p_kblk_w  the components, longest first {up to three blocks, their number | k << 8}
+    //   p_wpos, p_wfac  the Z values in that order, position q owning entries [p_wk[q],
+    //             p_wk[q + 1]): what the FP32 kernel forms the generators' W of
     //   p_sent    section entries of all levels: ma | centre of a middle row << 8 | exponent << 16
-    int4 *d_pz_unit = nullptr, *d_p_vent = nullptr, *d_p_lam = nullptr, *d_p_blk = nullptr, *d_p_kblk = nullptr;
+    int4 *d_pz_unit = nullptr, *d_p_vent = nullptr, *d_p_lam = nullptr, *d_p_blk = nullptr, *d_p_kblk_w = nullptr;
     double *d_pz_ca = nullptr, *d_pz_cb = nullptr;
     float *d_pz_ca32 = nullptr, *d_pz_cb32 = nullptr;
     double *d_p_fac = nullptr;

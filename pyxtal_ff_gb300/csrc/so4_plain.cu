@@ -31,9 +31,12 @@
 //
 // Measured on a GB300 (one pass with the neighbour list; before: one CTA per centre for
 // everything, dU by recursion, every lane of a warp computing the image's set-up): FP64, 32,000
-// Si atoms, 0.93 M images, lmax 4: 142.3 -> 30.0 ms; FP32, 16,232 atoms in 256 structures, lmax
-// 3: 2.91 -> 1.38 ms.  FP64 is bound by the FP64 pipe (91 % busy in k_plain_z, 80 % in k_plain_u)
-// and, in k_plain_d64, by latency at twelve warps per SM (pipe half busy).
+// Si atoms, 0.93 M images, lmax 4: 142.3 -> 26.1 ms (k_plain_d64 14.3, k_plain_z 7.9, k_plain_u
+// 3.2); FP32, 16,232 atoms in 256 structures, lmax 3: 2.92 -> 1.14 ms.  k_plain_z is bound by the
+// FP64 pipe (91 % busy), k_plain_u too (80 %); k_plain_d64 by latency at twelve warps per SM: of
+// a CTA's 263,000 cycles the digit products take 115,000 (integer and shared-memory work around
+// the matrix instructions), V 48,000, the rows 46,000 (FP64), the set-up beside the rounding of
+// Z' 25,000.
 #include <cstdio>
 
 #include <algorithm>
@@ -87,6 +90,11 @@ struct PlainArgs {
 constexpr int VI = 16;
 __device__ __forceinline__ int v_at(int e, int img) { return e * VI + (img ^ ((e & 3) << 1)); }
 
+// -x or x by the sign bit: a negation is an FP64 instruction otherwise
+__device__ __forceinline__ double flip(double x, int neg) {
+    return __hiloint2double(__double2hiint(x) ^ (neg << 31), __double2loint(x));
+}
+
 // V of n <= 16 images (Cayley-Klein parameters ck[4][32], from image c0 on), all levels.  Lanes
 // take (entry, image) pairs of a level, image fastest: the FP64 pipe (1/64 of the FP32 rate)
 // is what counts, and this leaves no lane idle.
@@ -102,20 +110,21 @@ __device__ __forceinline__ void plain_rows(const SmallTables &st, const int4 *__
         for (int t = tid; t < cnt; t += NT) {
             const int e = (int)(((unsigned)t * inv) >> 20), img = t - e * n;
             const int4 en = __ldg(vent + hb + e);
-            cx<double> v = mk<double>(0.0, 0.0);
-            if (en.x >= 0) {
-                const pc<double> p = V[v_at(en.x, img)];
-                cx<double> q = mk<double>(p.re, (en.z & 1) ? -p.im : p.im);
-                if (en.z & 2) q = mk<double>(-q.re, -q.im);
-                cmac(v, mk<double>(ck[c0 + img], ck[32 + c0 + img]), q);
-            }
+            const double ar = ck[c0 + img], ai = ck[32 + c0 + img], br = ck[64 + c0 + img], bi = ck[96 + c0 + img];
+            double re = 0.0, im = 0.0;
             if (en.y >= 0) {
                 const pc<double> p = V[v_at(en.y, img)];
-                cx<double> q = mk<double>(p.re, (en.z & 1) ? -p.im : p.im);
-                if (en.z & 4) q = mk<double>(-q.re, -q.im);
-                cmsub(v, mk<double>(ck[64 + c0 + img], ck[96 + c0 + img]), q);
+                const double pr = flip(p.re, en.z >> 2), pi = flip(p.im, (en.z >> 2) ^ (en.z & 1));
+                re = fma(bi, pi, -br * pr);
+                im = fma(-bi, pr, -br * pi);
             }
-            V[v_at(hb + e, img)] = {v.re, v.im};
+            if (en.x >= 0) {
+                const pc<double> p = V[v_at(en.x, img)];
+                const double pr = flip(p.re, (en.z >> 1) & 1), pi = flip(p.im, ((en.z >> 1) ^ en.z) & 1);
+                re = fma(ar, pr, fma(-ai, pi, re));
+                im = fma(ar, pi, fma(ai, pr, im));
+            }
+            V[v_at(hb + e, img)] = {re, im};
         }
     }
     __syncthreads();
@@ -231,13 +240,14 @@ __global__ void __launch_bounds__(256) k_plain_tile(PlainArgs<float> A) {
     }
 }
 
-// FP32: V of up to 32 images, lane = image, V[entry][33]; a warp takes a row of the level, the
+// FP32: V of up to 32 images, lane = image, V[entry][P]; a warp takes a row of the level, the
 // previous row's entry ma - 1 stays in registers, so an entry is one shared load, eight
 // multiply-adds and one store.
-constexpr int VP32 = 33;
+// Pitch of an entry: at 40, four consecutive entries x eight images fill the banks twice, evenly;
+// 33 where that does not fit (twol 11 and 12).
+__host__ __device__ inline int vp32(int nh) { return nh > 320 ? 33 : 40; }
 template <int NT>
-__device__ __forceinline__ void plain_rows32(const SmallTables &st, const float *ck, pc<float> *V) {
-    constexpr int P = VP32;
+__device__ __forceinline__ void plain_rows32(const SmallTables &st, const float *ck, pc<float> *V, int P) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const float ar = ck[lane], ai = ck[32 + lane], br = ck[64 + lane], bi = ck[96 + lane];
     if (wid == 0) V[lane] = {1.f, 0.f};
@@ -358,11 +368,16 @@ __global__ void __launch_bounds__(256) k_plain_b(PlainArgs<T> A) {
 }
 
 // ---------------------------------------------------------------- dB/dr
-// What the images of one pass need (warp 0, lane = image base + lane of n): Cayley-Klein
-// parameters, the 3 x 4 matrix q that takes (P0..P3) to t = dB/dr, and rv = (R_i + r) / vol
-// (r / vol for an image of the centre itself).  j is the image's neighbour (-1 past n).
+// What the images of one pass need (warp 0, lane = image base + lane of n): conj(a), conj(b),
+// the 3 x 4 matrix q that takes (P0..P3) to t = dB/dr, and rv = (R_i + r) / vol (r / vol for an
+// image of the centre itself).  j is the image's neighbour (-1 past n).
+// With n the unit vector, M = cos psi + i sin psi m . sigma, m = (-n_x, -n_y, n_z), and
+// X_c = i v_c . sigma, v_c = (gamma, beta, alpha):
+//   v_c = (psi' - sin cos / r) n_c m + (sin cos / r) D e_c + (sin^2 / r) m x D e_c,
+// D = diag(-1, -1, 1), psi' = dpsi/dr.
 template <typename T>
-__device__ __forceinline__ void plain_image(const PlainArgs<T> &A, int a, int m, bool in, T inv_vol, int j, CK<T> &c, T (&q)[12], T (&rv)[3]) {
+__device__ __forceinline__ void plain_image(const PlainArgs<T> &A, int a, int m, bool in, T inv_vol, int j, T (&ck)[4],
+                                            T (&q)[12], T (&rv)[3]) {
     T x = T(1), y = T(0), z = T(0), w = T(0);
     if (in) {
         x = (T)A.img_r[3 * m];
@@ -376,21 +391,41 @@ __device__ __forceinline__ void plain_image(const PlainArgs<T> &A, int a, int m,
         x = r = T(1);
         y = z = T(0);
     }
-    T sf, dsf;
+    T sf, dsf, sn, cs;
     cutoff_fn<T>(A.prm.cutoff_id, r, A.rc, sf, dsf);
-    make_ck<T, true>(x, y, z, r, A.psi_fac * r, c);
-    const T ri[3] = {x, y, z}, wd = w * dsf / r, ws = w * sf;
+    if (sizeof(T) == 8) {
+        double s_, c_;
+        sincos((double)(A.psi_fac * r), &s_, &c_);
+        sn = (T)s_;
+        cs = (T)c_;
+    } else {
+        float s_, c_;
+        sincosf((float)(A.psi_fac * r), &s_, &c_);
+        sn = (T)s_;
+        cs = (T)c_;
+    }
+    const T ir = T(1) / r, n[3] = {x * ir, y * ir, z * ir};
+    ck[0] = cs;
+    ck[1] = sn * n[2];
+    ck[2] = sn * n[1];
+    ck[3] = sn * n[0];
+    const T ws = w * sf, wd = w * dsf, sr = sn * ir;
+    const T u = ws * (sr * cs), v = ws * (sr * sn), p = fma(ws, A.psi_fac, -u);
+    const T md[3] = {-n[0], -n[1], n[2]};  // m
+    const T vm[3] = {v * md[0], v * md[1], v * md[2]};
+    const T cross[3][3] = {{T(0), -vm[2], vm[1]}, {vm[2], T(0), -vm[0]}, {vm[1], -vm[0], T(0)}};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const cx<T> da = c.cda[k], db = c.cdb[k];
-        const T al = c.ca.re * da.im - c.ca.im * da.re + c.cb.im * db.re - c.cb.re * db.im;
-        const T be = c.cb.re * da.re + c.cb.im * da.im - c.ca.re * db.re - c.ca.im * db.im;
-        const T ga = c.cb.im * da.re - c.cb.re * da.im - c.ca.re * db.im + c.ca.im * db.re;
-        q[4 * k] = wd * ri[k];
-        q[4 * k + 1] = ws * al;
-        q[4 * k + 2] = ws * be;
-        q[4 * k + 3] = ws * ga;
-        rv[k] = (j == a ? ri[k] : (T)A.pos[3 * a + k] + ri[k]) * inv_vol;
+        const T pk = p * n[k];
+        q[4 * k] = wd * n[k];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {  // alpha, beta, gamma = components 2, 1, 0 of v
+            T t = fma(pk, md[c], cross[k][c]);
+            if (c == k) t += (k < 2) ? -u : u;
+            q[4 * k + 3 - c] = t;
+        }
+        const T ri = (k == 0) ? x : (k == 1 ? y : z);
+        rv[k] = (j == a ? ri : (T)A.pos[3 * a + k] + ri) * inv_vol;
     }
 }
 
@@ -532,7 +567,6 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
     __shared__ int4 lamt[SO4_LDIM_MAX];
     __shared__ PlainRuns R;
     __shared__ int s_unit;
-    __shared__ double s_inv;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (tid == 0) st = A.st;
     if (tid <= A.st.twol) lamt[tid] = __ldg(A.lam + tid);
@@ -554,51 +588,99 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
     }
     __syncthreads();
 
+    const int m0 = A.img_ptr[a], m1 = A.img_ptr[a + 1], p0 = A.pair_ptr[a], ns = A.nsite[a];
+    const bool self_img = A.pair_img[ns] < A.pair_img[ns + 1];
+    int npair = 0;
+    // warp 0: the set-up of up to 32 images, and how they fall into pairs
+    auto setup = [&](int base, int n, int part) {
+        const int m = base + lane;
+        const int j = lane < n ? A.img_j[m] : -1;
+        const bool fresh = lane < n && (m == m0 || A.img_j[m - 1] != j);
+        double ck[4], q[12], rv[3];
+        plain_image<double>(A, a, m, lane < n, 1.0 / A.geom[A.astruct[a]].vol, j, ck, q, rv);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) par[32 * i + lane] = ck[i];
+#pragma unroll
+        for (int i = 0; i < 12; ++i) par[128 + 32 * i + lane] = q[i];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) par[512 + 32 * i + lane] = rv[i];
+        plain_runs(R, n, part, j, fresh, a, p0, self_img, npair);
+    };
     // ---- Z' as integers relative to each component's largest entry: the values into their
-    // slots and the components' exponents, then the integers in place
-    for (int q0 = 0; q0 < nz; q0 += DT) {
-        const int q = q0 + tid;
-        int ex = EMIN, k = -1;
-        if (q < nz) {
-            const pc<double> v = Zt[(size_t)q * 32];
-            ((pc<double> *)Zi)[q] = v;
-            const int ze = __ldg(A.zent + q), b = ze & 0xffff;
-            k = __ldg(&A.blk[b].x);
-            const int hf = __double2hiint(__ldg(A.fac + b));
-            const unsigned top = max((unsigned)__double2hiint(v.re) & 0x7fffffffu, (unsigned)__double2hiint(v.im) & 0x7fffffffu);
-            // f v 2^-row < 2^ex: the exponents, and one less where the leading 11 bits of the
-            // mantissas, rounded up, multiply to less than 2; Inf and NaN far above
-            const unsigned mant = (((top >> 10) & 0x3ff) + 0x401) * (((hf >> 10) & 0x3ff) + 0x401);
-            ex = top >= 0x7ff00000u ? KBAD : (int)(top >> 20) + (hf >> 20) - 2044 - (ze >> 16) - (mant < (1u << 21) ? 1 : 0);
+    // slots and the components' exponents (warps 1.., while warp 0 sets up the first images),
+    // then the integers in place
+    if (wid == 0) {
+        const int n = min(32, m1 - m0);
+        setup(m0, n, n > VI ? (n + 1) / 2 : n);
+    } else {
+        constexpr int NQ = DT - 32, RQ = 7;
+        for (int q0 = 0; q0 < nz; q0 += RQ * NQ) {
+            pc<double> v[RQ];
+            int ze[RQ];
+#pragma unroll
+            for (int r = 0; r < RQ; ++r) {
+                const int q = q0 + r * NQ + tid - 32;
+                ze[r] = q < nz ? __ldg(A.zent + q) : -1;
+                if (q < nz) v[r] = Zt[(size_t)q * 32];
+            }
+#pragma unroll
+            for (int r = 0; r < RQ; ++r) {
+                int ex = EMIN, k = -1;
+                if (ze[r] >= 0) {
+                    const int b = ze[r] & 0xffff;
+                    ((pc<double> *)Zi)[q0 + r * NQ + tid - 32] = v[r];
+                    k = __ldg(&A.blk[b].x);
+                    const int hf = __double2hiint(__ldg(A.fac + b));
+                    const unsigned top = max((unsigned)__double2hiint(v[r].re) & 0x7fffffffu,
+                                             (unsigned)__double2hiint(v[r].im) & 0x7fffffffu);
+                    // f v 2^-row < 2^ex: the exponents, and one less where the leading 11 bits of
+                    // the mantissas, rounded up, multiply to less than 2; Inf and NaN far above
+                    const unsigned mant = (((top >> 10) & 0x3ff) + 0x401) * (((hf >> 10) & 0x3ff) + 0x401);
+                    ex = top >= 0x7ff00000u
+                             ? KBAD
+                             : (int)(top >> 20) + (hf >> 20) - 2044 - (ze[r] >> 16) - (mant < (1u << 21) ? 1 : 0);
+                }
+                const unsigned peers = __match_any_sync(0xffffffffu, k);
+                const int big = __reduce_max_sync(peers, ex);
+                if (k >= 0 && lane == __ffs(peers) - 1) atomicMax(kex + k, big);
+            }
         }
-        const unsigned peers = __match_any_sync(0xffffffffu, k);
-        const int big = __reduce_max_sync(peers, ex);
-        if (k >= 0 && lane == __ffs(peers) - 1) atomicMax(kex + k, big);
     }
     __syncthreads();
     const int bz = ZB - A.cw;
     // P = integer x 2^(psh + kex), for g = 0 2^-cw less (W0 is Z' x 2^cw)
     const int psh = PSH - (VB - A.vs) - bz;
-    for (int q = tid; q < nz; q += DT) {
-        const pc<double> v = ((const pc<double> *)Zi)[q];
-        const int ze = __ldg(A.zent + q), b = ze & 0xffff;
-        const int4 bk = __ldg(A.blk + b);
-        const int ex = kex[bk.x];
-        const double f = __ldg(A.fac + b);
-        const double s = ex >= KBAD ? 0.0 : mul2(f, bz - ex - (ze >> 16));
-        longlong2 z;
-        z.x = __double2ll_rn(v.re * s);
-        z.y = __double2ll_rn(v.im * s);
-        Zi[q] = z;
-        if (bk.w == 0 && ex < KBAD) c00[bk.x] = __double2ll_rn(v.re * mul2(f, A.cw - psh - ex - 1));
+    for (int q0 = tid; q0 < nz; q0 += 4 * DT) {
+        pc<double> v[4];
+        int4 bk[4];
+        int ex[4], row[4];
+        double f[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int q = q0 + r * DT;
+            if (q >= nz) break;
+            const int ze = __ldg(A.zent + q), b = ze & 0xffff;
+            v[r] = ((const pc<double> *)Zi)[q];
+            bk[r] = __ldg(A.blk + b);
+            f[r] = __ldg(A.fac + b);
+            row[r] = ze >> 16;
+            ex[r] = kex[bk[r].x];
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int q = q0 + r * DT;
+            if (q >= nz) break;
+            const double s = ex[r] >= KBAD ? 0.0 : mul2(f[r], bz - ex[r] - row[r]);
+            longlong2 z;
+            z.x = __double2ll_rn(v[r].re * s);
+            z.y = __double2ll_rn(v[r].im * s);
+            Zi[q] = z;
+            if (bk[r].w == 0 && ex[r] < KBAD) c00[bk[r].x] = __double2ll_rn(v[r].re * mul2(f[r], A.cw - psh - ex[r] - 1));
+        }
     }
 
-    const int m0 = A.img_ptr[a], m1 = A.img_ptr[a + 1], p0 = A.pair_ptr[a], ns = A.nsite[a];
-    const bool self_img = A.pair_img[ns] < A.pair_img[ns + 1];
     const int nslot = DT / nB, slot = tid / nB, k = tid - slot * nB;
     double dsum[3] = {0.0, 0.0, 0.0};
-    int npair = 0;
-    if (tid == 0) s_inv = 1.0 / A.geom[A.astruct[a]].vol;
     // the (i, i) row takes the centre's own images as they come
     if (self_img && A.want_stress)
         for (int q = tid; q < 9 * nB; q += DT) A.rdxdr[(size_t)ns * nB * 9 + q] = 0.0;
@@ -610,24 +692,10 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
 
     for (int base = m0; base < m1; base += 32) {
         const int n = min(32, m1 - base), part = n > VI ? (n + 1) / 2 : n;
-        if (wid == 0) {
-            const int m = base + lane;
-            const int j = lane < n ? A.img_j[m] : -1;
-            const bool fresh = lane < n && (m == m0 || A.img_j[m - 1] != j);
-            CK<double> ck;
-            double q[12], rv[3];
-            plain_image<double>(A, a, m, lane < n, s_inv, j, ck, q, rv);
-            par[lane] = ck.ca.re;
-            par[32 + lane] = ck.ca.im;
-            par[64 + lane] = ck.cb.re;
-            par[96 + lane] = ck.cb.im;
-#pragma unroll
-            for (int i = 0; i < 12; ++i) par[128 + 32 * i + lane] = q[i];
-#pragma unroll
-            for (int i = 0; i < 3; ++i) par[512 + 32 * i + lane] = rv[i];
-            plain_runs(R, n, part, j, fresh, a, p0, self_img, npair);
+        if (base != m0) {
+            if (wid == 0) setup(base, n, part);
+            __syncthreads();
         }
-        __syncthreads();
         for (int h = 0; h * part < n; ++h) {
             const int c0 = h * part, nc = min(part, n - c0);
             plain_rows<DT>(st, A.vent, par, c0, nc, V);
@@ -635,15 +703,15 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
             // column tiles' ends
             const int sh = nc > 8 ? 4 : 3;
             for (int t = tid; t < nh << sh; t += DT) {
-                const int e = t >> sh, i = t & ((1 << sh) - 1);
+                const int e = t >> sh, i = t & ((1 << sh) - 1), at = v_at(e, i);
                 const int w = __ldg(&A.vent[e].w), ex = VB - A.vs + (w >> 16) - (w & 1);
                 longlong2 z = {0, 0};
                 if (i < nc) {
-                    const pc<double> v = V[v_at(e, i)];
+                    const pc<double> v = V[at];
                     z.x = __double2ll_rn(mul2(v.re, ex));
                     z.y = __double2ll_rn(mul2(v.im, ex));
                 }
-                Vi[v_at(e, i)] = z;
+                Vi[at] = z;
             }
             for (int q = tid; q < 8 * VI * CB; q += DT) Cl[q] = 0;
             if (tid == 0) s_unit = 0;
@@ -802,6 +870,7 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
         }
     }
     // ---- the (i, i) row: minus the sum of the others
+    const double inv_vol = 1.0 / A.geom[A.astruct[a]].vol;
     double *Ds = (double *)Cl;
     if (slot < nslot)
         for (int q = 0; q < 3; ++q) Ds[(slot * nB + k) * 3 + q] = dsum[q];
@@ -814,40 +883,47 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
             for (int w = 0; w < nslot; ++w) s += Ds[(w * nB + kk) * 3 + q];
             d[q] = -s;
         }
-        plain_self_row<double>(A, a, ns, kk, s_inv, d, self_img);
+        plain_self_row<double>(A, a, ns, kk, inv_vol, d, self_img);
     }
 }
 
-// FP32.  Lane = image throughout: the threads form W of a batch of components' entries in
-// shared memory, then a warp takes one component at a time, sums P_g over its entries (up to
-// 255) and forms t.
+// FP32.  The threads form W of a batch of components' entries in shared memory; then a warp
+// takes a component, its four groups of eight lanes every fourth entry and four images a lane:
+// six shared loads for 4 entries x 32 images (with an entry at a time and an image per lane it
+// was three loads of as many wavefronts for 1 x 32), and the groups' sums are exchanged so that
+// every lane ends with one image's P and forms its t.
 constexpr int ST = 256;     // threads
 constexpr int WCAP = 1024;  // entries of a batch: whole components, at least one
 
+// Batches of positions in the longest-first order of components: batch b holds [k[b], k[b + 1])
+struct PlainBatches {
+    int n, k[24];
+};
+
 struct D32Smem {
     int cb, wcap;  // pitch of a row of t: n_b rounded up to odd; entries of the W buffer
-    size_t t, w, par, total;
+    size_t t, w, vrow, par, total;
     __host__ __device__ D32Smem(int nh, int nz, int nB, int emax) {
         cb = nB | 1;
         wcap = nz < WCAP ? nz : (3 * emax > WCAP ? 3 * emax : WCAP);
         // V, and over it the warps' row buffers (9 floats per component) or partial (i, i) sums
-        const size_t v = sizeof(pc<float>) * (size_t)nh * VP32, s = sizeof(float) * 9 * (size_t)nB * (ST / 32);
+        const size_t v = sizeof(pc<float>) * (size_t)nh * vp32(nh), s = sizeof(float) * 9 * (size_t)nB * (ST / 32);
         w = ((v > s ? v : s) + 15) & ~(size_t)15;
-        t = w + sizeof(float) * 8 * (size_t)wcap;
-        par = t + ((sizeof(float) * 3 * 32 * (size_t)cb + 15) & ~(size_t)15);
+        vrow = w + sizeof(float) * 8 * (size_t)wcap;
+        t = vrow + sizeof(int) * (size_t)wcap;
+        par = t + sizeof(float) * 3 * 32 * (size_t)cb;
         total = (par + sizeof(float) * 32 * 19 + 15) & ~(size_t)15;
     }
 };
 
 // KS: components per lane in the row phase, 32 KS >= n_b
 template <int KS>
-__global__ void __launch_bounds__(ST) k_plain_d32(PlainArgs<float> A, int emax) {
-    constexpr int P = VP32;
+__global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<float> A, int emax, PlainBatches Bt) {
+    const int P = vp32(A.n_half);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ SmallTables st;
     __shared__ PlainRuns R;
     __shared__ int s_comp;
-    __shared__ float s_inv;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (tid == 0) st = A.st;
     const int nB = A.n_b, c = blockIdx.x, a = A.a0 + c;
@@ -855,11 +931,11 @@ __global__ void __launch_bounds__(ST) k_plain_d32(PlainArgs<float> A, int emax) 
     const int CB = L.cb;
     pc<float> *V = (pc<float> *)smem_raw;
     float4 *W = (float4 *)(smem_raw + L.w);
+    int *vrow = (int *)(smem_raw + L.vrow);
     float *t3 = (float *)(smem_raw + L.t), *par = (float *)(smem_raw + L.par);
     const pc<float> *Zt = A.zt + (size_t)(c >> 5) * A.n_z * 32 + (c & 31);
     const int m0 = A.img_ptr[a], m1 = A.img_ptr[a + 1], p0 = A.pair_ptr[a], ns = A.nsite[a];
     const bool self_img = A.pair_img[ns] < A.pair_img[ns + 1];
-    if (tid == 0) s_inv = (float)(1.0 / A.geom[A.astruct[a]].vol);
     // the (i, i) row takes the centre's own images as they come
     if (self_img && A.want_stress)
         for (int q = tid; q < 9 * nB; q += ST) A.rdxdr[(size_t)ns * nB * 9 + q] = 0.f;
@@ -867,84 +943,108 @@ __global__ void __launch_bounds__(ST) k_plain_d32(PlainArgs<float> A, int emax) 
 #pragma unroll
     for (int s = 0; s < KS; ++s) dsum[s][0] = dsum[s][1] = dsum[s][2] = 0.f;
     int npair = 0;
-    bool formed = false;  // W of every component is in the buffer (they fit) from the first pass on
+    // W of a batch's components, by threads t0.. of nt
+    auto form = [&](int b, int t0, int nt) {
+        const int w0 = __ldg(A.wk + Bt.k[b]), w1 = __ldg(A.wk + Bt.k[b + 1]);
+#pragma unroll 4
+        for (int e = w0 + t0; e < w1; e += nt) {
+            const int4 ps = __ldg(A.wpos + e);
+            const float4 f = __ldg(A.wfac + e);
+            const pc<float> z = Zt[(size_t)ps.x * 32], zq = Zt[(size_t)ps.z * 32];
+            pc<float> zn = Zt[(size_t)ps.y * 32];
+            if (ps.w & 1) zn.re = -zn.re;  // the mirror -conj(Z'[m-1]) past a middle row's centre
+            const float xr = f.z * zn.re, xi = f.z * zn.im, yr = f.w * zq.re, yi = f.w * zq.im;
+            // (re of W0..W3), (im of W0..W3)
+            W[2 * (e - w0)] = make_float4(f.x * z.re, f.y * z.im, xr - yr, xi + yi);
+            W[2 * (e - w0) + 1] = make_float4(f.x * z.im, -f.y * z.re, xi - yi, -(xr + yr));
+            vrow[e - w0] = (ps.w >> 1) * P;
+        }
+    };
+    auto setup = [&](int base, int n) {  // warp 0
+        const int m = base + lane;
+        const int j = lane < n ? A.img_j[m] : -1;
+        const bool fresh = lane < n && (m == m0 || A.img_j[m - 1] != j);
+        float ck[4], q[12], rv[3];
+        plain_image<float>(A, a, m, lane < n, (float)(1.0 / A.geom[A.astruct[a]].vol), j, ck, q, rv);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) par[32 * i + lane] = ck[i];
+#pragma unroll
+        for (int i = 0; i < 12; ++i) par[128 + 32 * i + lane] = q[i];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) par[512 + 32 * i + lane] = rv[i];
+        plain_runs(R, n, 32, j, fresh, a, p0, self_img, npair);
+    };
+    // the first images' set-up (warp 0) beside the first batch's W (the others)
+    if (wid == 0) setup(m0, min(32, m1 - m0));
+    else form(0, tid - 32, ST - 32);
+    int have = 0;  // the batch the buffer holds
+    const int sub = lane >> 3, il = lane & 7;
     __syncthreads();
 
     for (int base = m0; base < m1; base += 32) {
         const int n = min(32, m1 - base);
-        if (wid == 0) {
-            const int m = base + lane;
-            const int j = lane < n ? A.img_j[m] : -1;
-            const bool fresh = lane < n && (m == m0 || A.img_j[m - 1] != j);
-            CK<float> ck;
-            float q[12], rv[3];
-            plain_image<float>(A, a, m, lane < n, s_inv, j, ck, q, rv);
-            par[lane] = ck.ca.re;
-            par[32 + lane] = ck.ca.im;
-            par[64 + lane] = ck.cb.re;
-            par[96 + lane] = ck.cb.im;
-#pragma unroll
-            for (int i = 0; i < 12; ++i) par[128 + 32 * i + lane] = q[i];
-#pragma unroll
-            for (int i = 0; i < 3; ++i) par[512 + 32 * i + lane] = rv[i];
-            plain_runs(R, n, 32, j, fresh, a, p0, self_img, npair);
-        }
-        __syncthreads();
-        plain_rows32<ST>(st, par, V);
-        float qm[12];
-#pragma unroll
-        for (int i = 0; i < 12; ++i) qm[i] = par[128 + 32 * i + lane];
-        // ---- t of every component, a batch of components at a time
-        for (int k0 = 0; k0 < nB;) {
-            const int w0 = __ldg(A.wk + k0);
-            int k1 = k0 + 1;
-            while (k1 < nB && __ldg(A.wk + k1 + 1) - w0 <= L.wcap) ++k1;
-            if (!formed)
-                for (int e = w0 + tid; e < __ldg(A.wk + k1); e += ST) {
-                    const int4 ps = __ldg(A.wpos + e);
-                    const float4 f = __ldg(A.wfac + e);
-                    const pc<float> z = Zt[(size_t)ps.x * 32], zq = Zt[(size_t)ps.z * 32];
-                    pc<float> zn = Zt[(size_t)ps.y * 32];
-                    if (ps.w) zn.re = -zn.re;  // the mirror -conj(Z'[m-1]) past a middle row's centre
-                    const float xr = f.z * zn.re, xi = f.z * zn.im, yr = f.w * zq.re, yi = f.w * zq.im;
-                    // (re of W0..W3), (im of W0..W3)
-                    W[2 * (e - w0)] = make_float4(f.x * z.re, f.y * z.im, xr - yr, xi + yi);
-                    W[2 * (e - w0) + 1] = make_float4(f.x * z.im, -f.y * z.re, xi - yi, -(xr + yr));
-                }
-            formed = k0 == 0 && k1 == nB;
-            if (tid == 0) s_comp = k1 - 1;
+        if (base != m0) {
+            if (wid == 0) setup(base, n);
             __syncthreads();
-            for (;;) {  // the last components are the longest
-                int k = 0;
-                if (lane == 0) k = atomicSub(&s_comp, 1);
-                k = __shfl_sync(0xffffffffu, k, 0);
-                if (k < k0) break;
-                const int4 kb = __ldg(A.kblk + k);
-                const float4 *w = W + 2 * (__ldg(A.wk + k) - w0);
-                float2 p01 = make_float2(0.f, 0.f), p23 = p01;  // (P0, P1), (P2, P3)
-                for (int ib = 0; ib < kb.w; ++ib) {
-                    const int4 bk = __ldg(A.blk + (ib == 0 ? kb.x : (ib == 1 ? kb.y : kb.z)));
-                    const pc<float> *v = V + (size_t)st.h_block[bk.w] * P + lane;
-                    const int E = bk.z;
-#pragma unroll 4
-                    for (int e = 0; e < E; ++e) {
-                        const pc<float> u = v[e * P];
-                        const float4 wr = w[2 * e], wi = w[2 * e + 1];
+        }
+        plain_rows32<ST>(st, par, V, P);
+        float qm[12];  // of this lane's image, il + 8 sub = lane after the exchange below
+        const int img = 8 * sub + il;
+#pragma unroll
+        for (int i = 0; i < 12; ++i) qm[i] = par[128 + 32 * i + img];
+        // ---- t of every component, a batch of components at a time
+        for (int b = 0; b < Bt.n; ++b) {
+            if (have != b) {
+                form(b, tid, ST);
+                have = b;
+            }
+            const int w0 = __ldg(A.wk + Bt.k[b]), k1 = Bt.k[b + 1];
+            if (tid == 0) s_comp = Bt.k[b];
+            __syncthreads();
+            for (;;) {
+                int pos = 0;
+                if (lane == 0) pos = atomicAdd(&s_comp, 1);
+                pos = __shfl_sync(0xffffffffu, pos, 0);
+                if (pos >= k1) break;
+                const int e1 = __ldg(A.wk + pos + 1) - w0, kk = __ldg(&A.kblk[pos].w) >> 8;
+                float2 p01[4], p23[4];  // (P0, P1), (P2, P3) of images il + 8 i
+#pragma unroll
+                for (int i = 0; i < 4; ++i) p01[i] = p23[i] = make_float2(0.f, 0.f);
+#pragma unroll 2
+                for (int e = __ldg(A.wk + pos) - w0 + sub; e < e1; e += 4) {
+                    const float4 wr = W[2 * e], wi = W[2 * e + 1];
+                    const pc<float> *v = V + vrow[e] + il;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const pc<float> u = v[8 * i];
                         const float2 ur = make_float2(u.re, u.re), ui = make_float2(u.im, u.im);
-                        p01 = __ffma2_rn(ur, make_float2(wr.x, wr.y), p01);
-                        p23 = __ffma2_rn(ur, make_float2(wr.z, wr.w), p23);
-                        p01 = __ffma2_rn(ui, make_float2(wi.x, wi.y), p01);
-                        p23 = __ffma2_rn(ui, make_float2(wi.z, wi.w), p23);
+                        p01[i] = __ffma2_rn(ur, make_float2(wr.x, wr.y), p01[i]);
+                        p23[i] = __ffma2_rn(ur, make_float2(wr.z, wr.w), p23[i]);
+                        p01[i] = __ffma2_rn(ui, make_float2(wi.x, wi.y), p01[i]);
+                        p23[i] = __ffma2_rn(ui, make_float2(wi.z, wi.w), p23[i]);
                     }
-                    w += 2 * E;
                 }
+                // add the four groups' sums, each group keeping the images 8 sub ..
+                float2 a01[2], a23[2];
+                const bool up = sub & 2, odd = sub & 1;
+                auto swap2 = [](float2 keep, float2 give, int d) {
+                    keep.x += __shfl_xor_sync(0xffffffffu, give.x, d);
+                    keep.y += __shfl_xor_sync(0xffffffffu, give.y, d);
+                    return keep;
+                };
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    a01[i] = swap2(up ? p01[2 + i] : p01[i], up ? p01[i] : p01[2 + i], 16);
+                    a23[i] = swap2(up ? p23[2 + i] : p23[i], up ? p23[i] : p23[2 + i], 16);
+                }
+                const float2 s01 = swap2(odd ? a01[1] : a01[0], odd ? a01[0] : a01[1], 8);
+                const float2 s23 = swap2(odd ? a23[1] : a23[0], odd ? a23[0] : a23[1], 8);
 #pragma unroll
                 for (int q = 0; q < 3; ++q)
-                    t3[(q * 32 + lane) * CB + k] = fmaf(
-                        qm[4 * q], p01.x, fmaf(qm[4 * q + 1], p01.y, fmaf(qm[4 * q + 2], p23.x, qm[4 * q + 3] * p23.y)));
+                    t3[(q * 32 + img) * CB + kk] = fmaf(
+                        qm[4 * q], s01.x, fmaf(qm[4 * q + 1], s01.y, fmaf(qm[4 * q + 2], s23.x, qm[4 * q + 3] * s23.y)));
             }
             __syncthreads();
-            k0 = k1;
         }
         // ---- rows: a warp per pair, lane = component; whole lines through the warp's buffer
         float *buf = (float *)smem_raw + (size_t)9 * nB * wid;
@@ -1001,6 +1101,7 @@ __global__ void __launch_bounds__(ST) k_plain_d32(PlainArgs<float> A, int emax) 
         __syncthreads();
     }
     // ---- the (i, i) row: minus the sum of the others
+    const float inv_vol = (float)(1.0 / A.geom[A.astruct[a]].vol);
     float *Ds = (float *)smem_raw;
 #pragma unroll
     for (int s = 0; s < KS; ++s) {
@@ -1017,7 +1118,7 @@ __global__ void __launch_bounds__(ST) k_plain_d32(PlainArgs<float> A, int emax) 
             for (int w = 0; w < ST / 32; ++w) s += Ds[(w * nB + k) * 3 + q];
             d[q] = -s;
         }
-        plain_self_row<float>(A, a, ns, k, s_inv, d, self_img);
+        plain_self_row<float>(A, a, ns, k, inv_vol, d, self_img);
     }
 }
 
@@ -1086,7 +1187,7 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
     A.vent = t->d_p_vent;
     A.lam = t->d_p_lam;
     A.blk = t->d_p_blk;
-    A.kblk = t->d_p_kblk;
+    A.kblk = t->d_p_kblk_w;
     A.hfull = t->d_hfull;
     A.ca = (const T *)(sizeof(T) == 8 ? (const void *)t->d_pz_ca : (const void *)t->d_pz_ca32);
     A.cb = (const T *)(sizeof(T) == 8 ? (const void *)t->d_pz_cb : (const void *)t->d_pz_cb32);
@@ -1148,9 +1249,19 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
         } else {
             const int emax = section_count(t->twol);
             const size_t sm = D32Smem(t->n_half, t->n_pz, t->n_b, emax).total;
+            const int wcap = D32Smem(t->n_half, t->n_pz, t->n_b, emax).wcap;
+            PlainBatches bt;
+            bt.n = 0;
+            bt.k[0] = 0;
+            while (bt.k[bt.n] < t->n_b) {  // every component has at most 3 emax <= wcap entries
+                int k = bt.k[bt.n] + 1;
+                while (k < t->n_b && t->p_wk[k + 1] - t->p_wk[bt.k[bt.n]] <= wcap) ++k;
+                if (bt.n + 1 >= 23) return SO4_ERR_UNSUPPORTED;
+                bt.k[++bt.n] = k;
+            }
             auto kern = t->n_b <= 32 ? k_plain_d32<1> : (t->n_b <= 64 ? k_plain_d32<2> : (t->n_b <= 96 ? k_plain_d32<3> : k_plain_d32<5>));
             if ((rc = so4_set_smem((const void *)kern, sm))) return rc;
-            kern<<<n, ST, sm, st>>>(A, emax);
+            kern<<<n, ST, sm, st>>>(A, emax, bt);
         }
         so4_count_launch();
     }

@@ -103,7 +103,7 @@ void free_device(so4_tables *t) {
     cudaFree(t->d_p_fac);
     cudaFree(t->d_p_sent);
     cudaFree(t->d_p_bblk);
-    cudaFree(t->d_p_kblk);
+    cudaFree(t->d_p_kblk_w);
     cudaFree(t->d_p_zent);
     cudaFree(t->d_p_wpos);
     cudaFree(t->d_p_wfac);
@@ -392,11 +392,22 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
             if (blks[bi].z0 == bent[k].z[0]) p_bblk[k] = pblk_of[bi];
     // FP32: W0..W3 of a block's entry are (w.x Z', -i w.y Z', w.z Z'[m+1] - w.w Z'[m-1],
     // -i (w.z Z'[m+1] + w.w Z'[m-1])), with the block's factor and, at the centre of a middle
-    // row, the half weight inside; entries listed component by component
+    // row, the half weight inside; entries listed component by component, the longest first
     std::vector<int4> p_wpos;
     std::vector<float4> p_wfac;
     std::vector<int> p_wk(t->n_b + 1, 0);
+    // longest component first; position q holds component p_kblk_w[q].w >> 8
+    std::vector<int> kord(t->n_b), klen(t->n_b, 0);
+    std::vector<int4> p_kblk_w;
     for (int k = 0; k < t->n_b; ++k) {
+        const int bs[3] = {p_kblk[k].x, p_kblk[k].y, p_kblk[k].z};
+        kord[k] = k;
+        for (int i = 0; i < p_kblk[k].w; ++i) klen[k] += p_blk[bs[i]].z;
+    }
+    std::stable_sort(kord.begin(), kord.end(), [&](int x, int y) { return klen[x] > klen[y]; });
+    for (int q = 0; q < t->n_b; ++q) {
+        const int k = kord[q];
+        p_kblk_w.push_back(make_int4(p_kblk[k].x, p_kblk[k].y, p_kblk[k].z, p_kblk[k].w | (k << 8)));
         const int bs[3] = {p_kblk[k].x, p_kblk[k].y, p_kblk[k].z};
         for (int i = 0; i < p_kblk[k].w; ++i) {
             const int4 b = p_blk[bs[i]];
@@ -405,13 +416,14 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
                 const bool ctr = 2 * mb == b.w && 2 * ma == b.w;
                 const double f = p_fac[bs[i]] * (ctr ? 0.5 : 1.0);
                 // positions of Z', Z'[m+1], Z'[m-1] (past a row's end: Z' itself, weight 0), and
-                // whether Z'[m+1] is the mirror -conj(Z'[m-1])
+                // whether Z'[m+1] is the mirror -conj(Z'[m-1]) | the entry of V << 1
                 p_wpos.push_back(make_int4(b.y + e, b.y + e + (ctr ? (ma > 0 ? -1 : 0) : (ma < b.w ? 1 : 0)),
-                                           b.y + e - (ma > 0 ? 1 : 0), ctr ? 1 : 0));
+                                           b.y + e - (ma > 0 ? 1 : 0),
+                                           (ctr ? 1 : 0) | ((t->h_block[b.w] + e) << 1)));
                 p_wfac.push_back(make_float4((float)f, (float)(f * (b.w - 2 * ma)), (float)(f * (b.w - ma)), (float)(f * ma)));
             }
         }
-        p_wk[k + 1] = (int)p_wpos.size();
+        p_wk[q + 1] = (int)p_wpos.size();
     }
     // U entry (l, mb, ma) = conj(a) P[ma] - conj(b) P[ma - 1], P row mb of level l - 1, or its
     // mirror (-1)^(..) conj of row l - 1 - mb: {index of P[ma], of P[ma - 1] (-1: none),
@@ -856,12 +868,12 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     if (!rc) rc = upload(&t->d_p_fac, p_fac);
     if (!rc) rc = upload(&t->d_p_sent, p_sent);
     if (!rc) rc = upload(&t->d_p_bblk, p_bblk);
-    if (!rc) rc = upload(&t->d_p_kblk, p_kblk);
+    if (!rc) rc = upload(&t->d_p_kblk_w, p_kblk_w);
+    t->p_wk = p_wk;
     if (!rc) rc = upload(&t->d_p_zent, p_zent);
     if (!rc) rc = upload(&t->d_p_wpos, p_wpos);
     if (!rc) rc = upload(&t->d_p_wfac, p_wfac);
     if (!rc) rc = upload(&t->d_p_wk, p_wk);
-    t->p_wk = p_wk;
     if (!rc) rc = prc;
     if (!rc) rc = upload(&t->d_blk, blks);
     if (!rc) {
