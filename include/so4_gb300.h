@@ -187,7 +187,8 @@ int so4_nl_pairs(const so4_geom *d_geom, int nstruct, const int *d_atom_struct, 
  * atom of the workspace (so4_nl_workspace_size(natoms, nbins, natoms * slot_cap) bytes at
  * least).  An atom with more than slot_cap images sets status bits SO4_ERR_SLOTS and
  * SO4_ERR_CAPACITY; the largest per-atom count is left at ((int *)d_work)[8].
- * so4_nl_sort then does the rest of so4_nl_fill from those slots (same outputs). */
+ * so4_nl_sort then does the rest of so4_nl_fill from those slots (same outputs; no pair
+ * counts with d_pair_ptr NULL). */
 int so4_nl_count_keys(const so4_geom *d_geom, int nstruct, int nbins, const double *d_pos, const int *d_atom_struct,
                       int natoms, double rcut, int slot_cap, int32_t *d_img_ptr, void *d_work, size_t work_bytes,
                       void *stream);
@@ -365,6 +366,17 @@ int so4_adjoint_gather(int natoms, int nstruct, const int *d_atom_ptr, const int
                        const int32_t *d_img_rev, const double *d_img_r, const float *d_g,
                        const float *d_eatom, double *d_part, double *d_forces, double *d_virial,
                        double *d_energy, void *stream);
+/* so4_adjoint_gather with two more results: with d_bias[nstruct] f64 non-NULL energy[s] gets
+ * bias[s] added, and with d_vol[nstruct] and d_stress[nstruct*6] f64 non-NULL the stress
+ * -(virial / vol) x 160.21766208 (GPa) in the order xx yy zz xy xz yz. */
+int so4_adjoint_gather_stress(int natoms, int nstruct, const int *d_atom_ptr, const int32_t *d_img_ptr,
+                              const int32_t *d_img_rev, const double *d_img_r, const float *d_g,
+                              const float *d_eatom, double *d_part, double *d_forces, double *d_virial,
+                              double *d_energy, const double *d_bias, const double *d_vol, double *d_stress,
+                              void *stream);
+/* That stress of virials already there. */
+int so4_virial_stress(int nstruct, const double *d_virial, const double *d_vol, double *d_stress, void *stream);
+
 
 /* Forward and adjoint in one call for an energy linear in B (beta = dE/dB does not
  * depend on B, e.g. the reference's order-1 polynomial regression,

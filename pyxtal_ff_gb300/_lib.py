@@ -119,6 +119,9 @@ def lib():
         "so4_adjoint_deidrj32": (_i, [_vp, C.POINTER(Params), _i, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp]),
         "so4_gather_workspace_size": (_sz, [_i]),
         "so4_adjoint_gather": (_i, [_i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+        "so4_adjoint_gather_stress": (_i, [_i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                                           _vp]),
+        "so4_virial_stress": (_i, [_i, _vp, _vp, _vp, _vp]),
         "so4_launch_count": (C.c_longlong, []),
         "so4_set_pdl": (C.c_int, [C.c_int]),
         "so4_peak_fma": (_i, [_i, _i, _i, _vp, C.POINTER(C.c_double), _vp]),

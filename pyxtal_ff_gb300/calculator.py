@@ -178,7 +178,7 @@ class SO4Calculator:
             x, forces, virial, energy = engine.adjoint_linear32(self.tables, self.params, nb, self._w_nb,
                                                                 self._w_site, beta, workspace=self._ws)
             energy = energy + self._counts @ model.bias.detach().double()
-            stress = -(virial.reshape(-1, 9)[:, VOIGT] / self._vol[:, None]) * EV_A3_TO_GPA
+            stress = engine.virial_stress(virial, self._vol)
             return dict(energy=energy, forces=forces, virial=virial, stress=stress, x=x, neighbors=nb)
         x, utot = engine.forward32(self.tables, self.params, nb, self._w_nb, self._w_site)
         xg = x.detach().requires_grad_(True)
@@ -187,7 +187,7 @@ class SO4Calculator:
             beta, = torch.autograd.grad(e_atom.sum(), xg)
         forces, virial, energy = engine.adjoint32(self.tables, self.params, nb, self._w_nb, utot, beta,
                                                   eatom=e_atom.detach())
-        stress = -(virial.reshape(-1, 9)[:, VOIGT] / self._vol[:, None]) * EV_A3_TO_GPA
+        stress = engine.virial_stress(virial, self._vol)
         return dict(energy=energy, forces=forces, virial=virial, stress=stress, x=x, neighbors=nb,
                     energies=e_atom.detach())
 
@@ -269,8 +269,6 @@ class CapturedStep:
         L = engine.lib()
         tab = calc.tables
         if self.linear:
-            self.ws = torch.empty(L.so4_linear_workspace_size(tab.handle, N, self.cap_m), dtype=torch.uint8,
-                                  device=dev)
             self.beta = model.coef.detach()[calc._species].to(torch.float32).contiguous()
             self.bias_s = (calc._counts @ model.bias.detach().double()).contiguous()
         else:
@@ -279,46 +277,37 @@ class CapturedStep:
             # a model with species_index() gets the atoms of each species precomputed
             self.model = model
             self.index = model.species_index(calc._species) if hasattr(model, "species_index") else None
-            nh = tab.n_half
             self.fws = torch.empty(max(L.so4_forward32_workspace_size(tab.handle, N), 1), dtype=torch.uint8,
                                    device=dev)
-            self.utot = torch.empty((max(N, 1), nh, 2), dtype=torch.float32, device=dev)
-            self.ybuf = torch.empty((max(N, 1), nh, 2), dtype=torch.float32, device=dev)
             self.beta = torch.empty((max(N, 1), tab.nB), dtype=torch.float32, device=dev)
-            self.eatom = torch.empty(max(N, 1), dtype=torch.float32, device=dev)
             self.energies = torch.empty(max(N, 1), dtype=torch.float64, device=dev)
-            self.g = torch.empty((self.cap_m, 3), dtype=torch.float32, device=dev)
-            self.part = torch.empty(L.so4_gather_workspace_size(N), dtype=torch.uint8, device=dev)
+        nh = tab.n_half
+        self.utot = torch.empty((max(N, 1), nh, 2), dtype=torch.float32, device=dev)
+        self.ybuf = torch.empty((max(N, 1), nh, 2), dtype=torch.float32, device=dev)
+        self.eatom = torch.empty(max(N, 1), dtype=torch.float32, device=dev)
+        self.g = torch.empty((self.cap_m, 3), dtype=torch.float32, device=dev)
+        self.part = torch.empty(L.so4_gather_workspace_size(N), dtype=torch.uint8, device=dev)
         self.x = torch.empty((max(N, 1), tab.nB), dtype=torch.float32, device=dev)
-        self.forces = torch.empty((max(N, 1), 3), dtype=torch.float64, device=dev)
+        # energy, forces and stress in one buffer, so that host_io copies them out together
+        self.out = torch.empty(S + 3 * N + 6 * S, dtype=torch.float64, device=dev)
+        self.energy, self.forces, self.stress = self._parts(self.out)
         self.virial = torch.empty((max(S, 1), 3, 3), dtype=torch.float64, device=dev)
-        self.energy_sum = torch.empty(max(S, 1), dtype=torch.float64, device=dev)
         # Branches: after the neighbour list every stage up to the gather is independent per
         # centre, so consecutive ranges of atoms (cut at multiples of 32) run as parallel graph
         # branches and the tail of one branch's kernels overlaps the others' work.
         self.branches = max(1, min(int(branches), N // 128)) if self.linear else 1
-        if self.branches > 1:
-            cuts = [0] + [min(N, (N * k // self.branches + 31) // 32 * 32) for k in range(1, self.branches)] + [N]
-            self.chunks = [(a0, a1) for a0, a1 in zip(cuts[:-1], cuts[1:]) if a1 > a0]
-            self.branches = len(self.chunks)
-            nh = tab.n_half
-            self.utot = torch.empty((N, nh, 2), dtype=torch.float32, device=dev)
-            self.ybuf = torch.empty((N, nh, 2), dtype=torch.float32, device=dev)
+        cuts = [0] + [min(N, (N * k // self.branches + 31) // 32 * 32) for k in range(1, self.branches)] + [N]
+        self.chunks = [(a0, a1) for a0, a1 in zip(cuts[:-1], cuts[1:]) if a1 > a0]
+        self.branches = max(1, len(self.chunks))
+        if self.linear:
             self.bc = [torch.empty((max(tab.n_bsec, 1), a1 - a0), dtype=torch.float32, device=dev)
                        for a0, a1 in self.chunks]
-            self.eatom = torch.empty(N, dtype=torch.float32, device=dev)
-            self.g = torch.empty((self.cap_m, 3), dtype=torch.float32, device=dev)
-            self.part = torch.empty(L.so4_gather_workspace_size(N), dtype=torch.uint8, device=dev)
-            self.sides = [torch.cuda.Stream(device=dev) for _ in range(self.branches - 1)]
-        self.energy = torch.empty(max(S, 1), dtype=torch.float64, device=dev)
-        self.stress = torch.empty((max(S, 1), 6), dtype=torch.float64, device=dev)
-        self._voigt = torch.tensor(VOIGT, device=dev)  # on the device before capture (no copies inside it)
+        self.sides = [torch.cuda.Stream(device=dev) for _ in range(self.branches - 1)]
         self.host_io = bool(host_io)
         if self.host_io:
             self.host_positions = torch.from_numpy(np.ascontiguousarray(batch.positions, dtype=np.float64)).pin_memory()
-            self.host_out = dict(energy=torch.empty(S, dtype=torch.float64).pin_memory(),
-                                 forces=torch.empty((N, 3), dtype=torch.float64).pin_memory(),
-                                 stress=torch.empty((S, 6), dtype=torch.float64).pin_memory())
+            self._host = torch.empty(self.out.shape, dtype=torch.float64).pin_memory()
+            self.host_out = dict(zip(("energy", "forces", "stress"), self._parts(self._host)))
         self.launches = 0
         # eager warm-up on a side stream (sets kernel attributes, lets torch's allocator settle)
         side = torch.cuda.Stream(device=dev)
@@ -345,31 +334,43 @@ class CapturedStep:
                 self._enqueue_linear()
             finally:
                 L.so4_set_pdl(prev)
-        if self.host_io:  # and the results back to the pinned host buffers
-            N, S = self.layout.natoms, self.layout.nstruct
-            self.host_out["energy"].copy_(self.energy[:S], non_blocking=True)
-            self.host_out["forces"].copy_(self.forces[:N], non_blocking=True)
-            self.host_out["stress"].copy_(self.stress[:S], non_blocking=True)
+        if self.host_io:  # and the results back to the pinned host buffer
+            self._host.copy_(self.out, non_blocking=True)
+
+    def _parts(self, buf):
+        """Views of energy (S,), forces (N, 3) and stress (S, 6) in one buffer."""
+        N, S = self.layout.natoms, self.layout.nstruct
+        return buf[:S], buf[S:S + 3 * N].view(N, 3), buf[S + 3 * N:].view(S, 6)
 
     def _enqueue_linear(self):
         lay, calc, tab, L = self.layout, self.calc, self.calc.tables, engine.lib()
         b = self.nl
         _p = engine._ptr
         check = engine.check
+        N, S_ = lay.natoms, lay.nstruct
+
+        def compute(a0, a1, bc):
+            """U_tot, B and Y, and the per-image dE/dr of one range of centres."""
+            n, s_ = a1 - a0, engine._stream()
+            check(L.so4_utot32(tab.handle, C.byref(calc.params), n, _p(calc._w_nb), _p(calc._w_site[a0:a1]),
+                               _p(b.img_ptr[a0:a1 + 1]), _p(b.img_j), _p(b.img_r), _p(self.utot[a0:a1]), s_),
+                  "so4_utot32")
+            check(L.so4_linear_by32(tab.handle, n, _p(self.utot[a0:a1]), _p(self.beta[a0:a1]), _p(self.x[a0:a1]),
+                                    _p(self.ybuf[a0:a1]), _p(bc), _p(self.eatom[a0:a1]), s_), "so4_linear_by32")
+            check(L.so4_adjoint_deidrj32(tab.handle, C.byref(calc.params), n, _p(calc._w_nb),
+                                         _p(b.img_ptr[a0:a1 + 1]), _p(b.img_j), _p(b.img_r), self.cap_m,
+                                         _p(self.ybuf[a0:a1]), _p(self.g), s_), "so4_adjoint_deidrj32")
+
         if self.branches == 1:
-            engine.enqueue_neighbors(lay, self.pos, b, lite=True)
-            check(L.so4_adjoint_linear32(tab.handle, C.byref(calc.params), lay.nstruct, _p(lay.atom_struct),
-                                         _p(lay.atom_ptr_dev), lay.natoms, _p(calc._w_nb), _p(calc._w_site),
-                                         _p(b.img_ptr), _p(b.img_j), _p(b.img_r), _p(b.img_rev), self.cap_m,
-                                         _p(self.beta), _p(self.x), _p(self.forces), _p(self.virial),
-                                         _p(self.energy_sum), _p(self.ws), self.ws.numel(), engine._stream()),
-                  "so4_adjoint_linear32")
+            engine.enqueue_neighbors(lay, self.pos, b, lite=True, count_pairs=False)
+            for (a0, a1), bc in zip(self.chunks, self.bc):
+                compute(a0, a1, bc)
         else:
             # the list itself runs per branch: bins for all atoms, then each branch counts and
             # sorts its own centres (their scans chained in branch order) and goes on to its
             # compute while the other branches' lists are still being built; the reverse images
             # (read only by the gather) and the summary follow the join
-            N, S_, G = lay.natoms, lay.nstruct, lay.nbins
+            G = lay.nbins
             check(L.so4_nl_bins(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N, b.slot_cap, _p(b.ws),
                                 b.ws.numel(), engine._stream()), "so4_nl_bins")
             main = torch.cuda.current_stream()
@@ -379,7 +380,6 @@ class CapturedStep:
             for (a0, a1), bc, st in zip(self.chunks, self.bc, [main] + self.sides):
                 with torch.cuda.stream(st):
                     s_ = engine._stream()
-                    n = a1 - a0
                     check(L.so4_nl_count_keys_range(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N,
                                                     lay.rcut, b.slot_cap, a0, a1, _p(b.ws), b.ws.numel(), s_),
                           "so4_nl_count_keys_range")
@@ -392,15 +392,7 @@ class CapturedStep:
                     check(L.so4_nl_sort_range(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N, a0, a1,
                                               _p(b.img_ptr), b.cap_m, b.slot_cap, _p(b.img_j), _p(b.img_off),
                                               _p(b.img_r), _p(b.ws), b.ws.numel(), s_), "so4_nl_sort_range")
-                    check(L.so4_utot32(tab.handle, C.byref(calc.params), n, _p(calc._w_nb), _p(calc._w_site[a0:a1]),
-                                       _p(b.img_ptr[a0:a1 + 1]), _p(b.img_j), _p(b.img_r), _p(self.utot[a0:a1]),
-                                       s_), "so4_utot32")
-                    check(L.so4_linear_by32(tab.handle, n, _p(self.utot[a0:a1]), _p(self.beta[a0:a1]),
-                                            _p(self.x[a0:a1]), _p(self.ybuf[a0:a1]), _p(bc), _p(self.eatom[a0:a1]),
-                                            s_), "so4_linear_by32")
-                    check(L.so4_adjoint_deidrj32(tab.handle, C.byref(calc.params), n, _p(calc._w_nb),
-                                                 _p(b.img_ptr[a0:a1 + 1]), _p(b.img_j), _p(b.img_r), self.cap_m,
-                                                 _p(self.ybuf[a0:a1]), _p(self.g), s_), "so4_adjoint_deidrj32")
+                    compute(a0, a1, bc)
             for sd in self.sides:
                 main.wait_stream(sd)
             check(L.so4_nl_pairs(_p(lay.geom), S_, _p(lay.atom_struct), N, _p(b.img_ptr), b.cap_m, _p(b.img_j),
@@ -408,13 +400,16 @@ class CapturedStep:
                                  _p(b.img_rev), _p(b.ws), b.ws.numel(), engine._stream()), "so4_nl_pairs")
             check(L.so4_nl_summary(_p(b.img_ptr), _p(None), N, _p(b.ws), b.ws.numel(), engine._stream(), None),
                   "so4_nl_summary")
-            check(L.so4_adjoint_gather(lay.natoms, lay.nstruct, _p(lay.atom_ptr_dev), _p(b.img_ptr), _p(b.img_rev),
-                                       _p(b.img_r), _p(self.g), _p(self.eatom), _p(self.part), _p(self.forces),
-                                       _p(self.virial), _p(self.energy_sum), engine._stream()), "so4_adjoint_gather")
-        S = lay.nstruct
-        torch.add(self.energy_sum[:S], self.bias_s, out=self.energy[:S])
-        # same operations as the uncaptured path, so the two agree bit for bit
-        self.stress[:S].copy_(-(self.virial[:S].reshape(S, 9)[:, self._voigt] / self.calc._vol[:, None]) * EV_A3_TO_GPA)
+        self._gather(self.bias_s)
+
+    def _gather(self, bias):
+        """Forces, virial, energy (plus the per-structure constant) and stress, with the arithmetic of
+        the uncaptured path (so4_virial_stress), so the two agree bit for bit."""
+        lay, b, _p = self.layout, self.nl, engine._ptr
+        engine.check(engine.lib().so4_adjoint_gather_stress(
+            lay.natoms, lay.nstruct, _p(lay.atom_ptr_dev), _p(b.img_ptr), _p(b.img_rev), _p(b.img_r), _p(self.g),
+            _p(self.eatom), _p(self.part), _p(self.forces), _p(self.virial), _p(self.energy), _p(bias),
+            _p(self.calc._vol), _p(self.stress), engine._stream()), "so4_adjoint_gather_stress")
 
     def _enqueue_model(self):
         """The general-model step: neighbour list, U_tot and B (so4_forward32), the model and
@@ -423,7 +418,7 @@ class CapturedStep:
         lay, calc, tab, L = self.layout, self.calc, self.calc.tables, engine.lib()
         b, _p, check, st = self.nl, engine._ptr, engine.check, engine._stream()
         N, S = lay.natoms, lay.nstruct
-        engine.enqueue_neighbors(lay, self.pos, b, lite=True)
+        engine.enqueue_neighbors(lay, self.pos, b, lite=True, count_pairs=False)
         check(L.so4_forward32(tab.handle, C.byref(calc.params), N, _p(calc._w_nb), _p(calc._w_site), _p(b.img_ptr),
                               _p(b.img_j), _p(b.img_r), _p(self.utot), _p(self.x), _p(self.fws), self.fws.numel(), st),
               "so4_forward32")
@@ -441,10 +436,7 @@ class CapturedStep:
         check(L.so4_adjoint_deidrj32(tab.handle, C.byref(calc.params), N, _p(calc._w_nb), _p(b.img_ptr),
                                      _p(b.img_j), _p(b.img_r), self.cap_m, _p(self.ybuf), _p(self.g), st),
               "so4_adjoint_deidrj32")
-        check(L.so4_adjoint_gather(N, S, _p(lay.atom_ptr_dev), _p(b.img_ptr), _p(b.img_rev), _p(b.img_r), _p(self.g),
-                                   _p(self.eatom), _p(self.part), _p(self.forces), _p(self.virial),
-                                   _p(self.energy), st), "so4_adjoint_gather")
-        self.stress[:S].copy_(-(self.virial[:S].reshape(S, 9)[:, self._voigt] / calc._vol[:, None]) * EV_A3_TO_GPA)
+        self._gather(None)
 
     def __call__(self, positions=None):
         """One step; positions (N,3) f64 from the host (pinned for an asynchronous copy)
@@ -466,8 +458,7 @@ class CapturedStep:
             self.pos.copy_(positions, non_blocking=True)
         self.graph.replay()
         N, S = self.layout.natoms, self.layout.nstruct
-        out = dict(energy=self.energy[:S], forces=self.forces[:N], virial=self.virial[:S], stress=self.stress[:S],
-                   x=self.x[:N])
+        out = dict(energy=self.energy, forces=self.forces, virial=self.virial[:S], stress=self.stress, x=self.x[:N])
         if not self.linear:
             out["energies"] = self.energies[:N]
         return out

@@ -1217,14 +1217,20 @@ __global__ void __launch_bounds__(GCH * GSUB) k_gather_fv(int natoms, int nstruc
     }
 }
 
-// One CTA per structure: virial[s] (9) and energy[s] from the head atoms and the chunk partials.
+// One virial component (eV) over a volume (A^3) as the reference's stress in GPa.
+__device__ __forceinline__ double stress_gpa(double virial, double vol) { return -(virial / vol) * 160.21766208; }
+
+// One CTA per structure: virial[s] (9) and energy[s] from the head atoms and the chunk partials;
+// with them, where asked for, the energy's constant and the stress.
 constexpr int GSS = GCH * GSUB;  // threads of the structure pass: one group per possible head atom
 __global__ void __launch_bounds__(GSS) k_struct_sum(const int *__restrict__ atom_ptr,
                                                    const int32_t *__restrict__ img_ptr,
                                                    const int32_t *__restrict__ img_rev,
                                                    const double *__restrict__ img_r, const float *__restrict__ g,
                                                    const float *__restrict__ eatom, const double *__restrict__ part,
-                                                   double *__restrict__ virial, double *__restrict__ energy) {
+                                                   double *__restrict__ virial, double *__restrict__ energy,
+                                                   const double *__restrict__ bias, const double *__restrict__ vol,
+                                                   double *__restrict__ stress) {
     constexpr int NSLOT = GSS / GPART;
     __shared__ float hv[GCH][GPART];
     __shared__ double red[NSLOT][GPART];
@@ -1255,11 +1261,23 @@ __global__ void __launch_bounds__(GSS) k_struct_sum(const int *__restrict__ atom
         double tot = 0.0;
         for (int k = 0; k < GCH; ++k) tot += (double)hv[k][t];
         for (int k = 0; k < NSLOT; ++k) tot += red[k][t];
-        if (t < 9)
+        if (t < 9) {
             virial[9 * (size_t)s + t] = tot;
-        else if (energy)
-            energy[s] = tot;
+            // xx yy zz xy xz yz of the row-major virial (components 0 4 8 1 2 5)
+            const int v = (t & 3) == 0 ? t / 4 : (t == 1 ? 3 : (t == 2 ? 4 : (t == 5 ? 5 : -1)));
+            if (stress && v >= 0) stress[6 * (size_t)s + v] = stress_gpa(tot, vol[s]);
+        } else if (energy) {
+            energy[s] = bias ? tot + bias[s] : tot;
+        }
     }
+}
+
+__global__ void k_stress(int nstruct, const double *__restrict__ virial, const double *__restrict__ vol,
+                         double *__restrict__ stress) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, s = i / 6, v = i - 6 * s;
+    if (s >= nstruct) return;
+    const int c = (v < 3) ? 4 * v : (v == 5 ? 5 : v - 2);
+    stress[i] = stress_gpa(virial[9 * (size_t)s + c], vol[s]);
 }
 
 size_t rootpq_floats(int ldim) { return (size_t)((ldim * ldim + 1) & ~1); }
@@ -1520,15 +1538,17 @@ extern "C" size_t so4_gather_workspace_size(int natoms) {
     return natoms < 0 ? 0 : sizeof(double) * gather_part_doubles(natoms);
 }
 
-extern "C" int so4_adjoint_gather(int natoms, int nstruct, const int *d_atom_ptr, const int32_t *d_img_ptr,
-                                  const int32_t *d_img_rev, const double *d_img_r, const float *d_g,
-                                  const float *d_eatom, double *d_part, double *d_forces, double *d_virial,
-                                  double *d_energy, void *stream) {
+extern "C" int so4_adjoint_gather_stress(int natoms, int nstruct, const int *d_atom_ptr, const int32_t *d_img_ptr,
+                                         const int32_t *d_img_rev, const double *d_img_r, const float *d_g,
+                                         const float *d_eatom, double *d_part, double *d_forces, double *d_virial,
+                                         double *d_energy, const double *d_bias, const double *d_vol, double *d_stress,
+                                         void *stream) {
     if (natoms < 0 || nstruct < 0) return SO4_ERR_ARG;
     if (natoms > 0 && (!d_atom_ptr || !d_img_ptr || !d_img_rev || !d_img_r || !d_g || !d_part || !d_forces))
         return SO4_ERR_ARG;
     if (nstruct > 0 && !d_virial) return SO4_ERR_ARG;
     if (natoms > 0 && nstruct == 0) return SO4_ERR_ARG;
+    if (d_stress && nstruct > 0 && !d_vol) return SO4_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     if (natoms > 0) {
         k_gather_fv<<<(natoms + GCH - 1) / GCH, GCH * GSUB, 0, st>>>(natoms, nstruct, d_atom_ptr, d_img_ptr, d_img_rev,
@@ -1537,9 +1557,27 @@ extern "C" int so4_adjoint_gather(int natoms, int nstruct, const int *d_atom_ptr
     }
     if (nstruct > 0) {
         k_struct_sum<<<nstruct, GSS, 0, st>>>(d_atom_ptr, d_img_ptr, d_img_rev, d_img_r, d_g, d_eatom, d_part,
-                                              d_virial, d_energy);
+                                              d_virial, d_energy, d_bias, d_vol, d_stress);
         so4_count_launch();
     }
+    return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
+}
+
+extern "C" int so4_adjoint_gather(int natoms, int nstruct, const int *d_atom_ptr, const int32_t *d_img_ptr,
+                                  const int32_t *d_img_rev, const double *d_img_r, const float *d_g,
+                                  const float *d_eatom, double *d_part, double *d_forces, double *d_virial,
+                                  double *d_energy, void *stream) {
+    return so4_adjoint_gather_stress(natoms, nstruct, d_atom_ptr, d_img_ptr, d_img_rev, d_img_r, d_g, d_eatom, d_part,
+                                     d_forces, d_virial, d_energy, nullptr, nullptr, nullptr, stream);
+}
+
+extern "C" int so4_virial_stress(int nstruct, const double *d_virial, const double *d_vol, double *d_stress,
+                                 void *stream) {
+    if (nstruct < 0 || (nstruct > 0 && (!d_virial || !d_vol || !d_stress))) return SO4_ERR_ARG;
+    if (nstruct == 0) return SO4_OK;
+    const int64_t n = 6 * (int64_t)nstruct;
+    k_stress<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(nstruct, d_virial, d_vol, d_stress);
+    so4_count_launch();
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
 }
 

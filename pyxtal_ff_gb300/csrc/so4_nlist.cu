@@ -24,6 +24,7 @@ constexpr int OFF_MAX = 511;
 
 struct NLWork {
     int *status;
+    size_t clear;    // bytes from status on that a new list starts from zero
     int *bin_cnt;    // nbins + 1
     int *bin_start;  // nbins + 1
     int *bin_cur;    // nbins
@@ -50,8 +51,9 @@ size_t carve(NLWork &w, void *base, int natoms, int nbins, int64_t nimg) {
     };
     w.status = (int *)take(SO4_WS_HEADER);
     w.bin_cnt = (int *)take(sizeof(int) * (nbins + 1));
-    w.bin_start = (int *)take(sizeof(int) * (nbins + 1));
     w.bin_cur = (int *)take(sizeof(int) * (nbins + 1));
+    w.clear = off;  // header and bin counters, cleared together
+    w.bin_start = (int *)take(sizeof(int) * (nbins + 1));
     w.bin_atoms = (int *)take(sizeof(int) * (natoms + 1));
     w.atom_bin = (int *)take(sizeof(int) * (natoms + 1));
     w.atom_shift = (int4 *)take(sizeof(int4) * (natoms + 1));
@@ -94,9 +96,9 @@ __device__ __noinline__ bool exact_inside(const so4_geom &g, const double *pi, c
     return norm_rn(r) < rcut;
 }
 
-__global__ void k_bin(const so4_geom *geom, const double *pos, const int *astruct, int natoms, NLWork w) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= natoms) return;
+// Bin, wrapping shift and FP32 position of atom a; returns its bin.
+__device__ __forceinline__ int bin_atom(const so4_geom *geom, const double *pos, const int *astruct, int a,
+                                        const NLWork &w) {
     const so4_geom &g = geom[astruct[a]];
     const double r[3] = {pos[3 * a], pos[3 * a + 1], pos[3 * a + 2]};
     if (!isfinite(r[0]) || !isfinite(r[1]) || !isfinite(r[2])) flag(w.status, SO4_ERR_NONFINITE);
@@ -121,7 +123,13 @@ __global__ void k_bin(const so4_geom *geom, const double *pos, const int *astruc
     const int bin = g.bin_base + (b[0] * g.nbin[1] + b[1]) * g.nbin[2] + b[2];
     w.atom_bin[a] = bin;
     w.pos32[a] = make_float4((float)r[0], (float)r[1], (float)r[2], 0.f);
-    atomicAdd(&w.bin_cnt[bin], 1);
+    return bin;
+}
+
+__global__ void k_bin(const so4_geom *geom, const double *pos, const int *astruct, int natoms, NLWork w) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= natoms) return;
+    atomicAdd(&w.bin_cnt[bin_atom(geom, pos, astruct, a, w)], 1);
 }
 
 __global__ void k_bin_fill(const int *astruct, int natoms, NLWork w) {
@@ -188,32 +196,88 @@ __global__ void __launch_bounds__(1024) k_scan(const int *in, int *out, int n, i
     if (t == 0) out[n] = carry_s;
 }
 
+// The bins of a small list (natoms <= BIN_ATOMS, nbins <= BIN_BINS) by one CTA: header cleared,
+// atoms binned (thread = atom), bin starts scanned and filled, in one launch instead of a
+// clear and three kernels.  Its FP64 work (about 30 operations per atom, 2 per cycle and SM)
+// stays below the latencies that it saves: 64 atoms 5.1 us instead of 9.9, 1,000 atoms 12.0
+// instead of 13.1 (sums of the kernels; each launch also has a gap of about 1 us).
+constexpr int BIN_ATOMS = 1024, BIN_BINS = 4096;
+__global__ void __launch_bounds__(1024) k_bin_small(const so4_geom *geom, const double *pos, const int *astruct,
+                                                    int natoms, int nbins, NLWork w) {
+    __shared__ int cnt[BIN_BINS], wsum[32];
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    if (t < SO4_WS_HEADER / 4) w.status[t] = 0;
+    for (int q = t; q < nbins; q += 1024) cnt[q] = 0;
+    __syncthreads();
+    int bin = 0, slot = 0;
+    if (t < natoms) {
+        bin = bin_atom(geom, pos, astruct, t, w);
+        slot = atomicAdd(cnt + bin, 1);
+    }
+    __syncthreads();
+    int v[4], tot = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        v[q] = (4 * t + q < nbins) ? cnt[4 * t + q] : 0;
+        tot += v[q];
+    }
+    int inc = tot;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += y;
+    }
+    if (lane == 31) wsum[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+        const int x = wsum[lane];
+        int winc = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, winc, d);
+            if (lane >= d) winc += y;
+        }
+        wsum[lane] = winc - x;
+    }
+    __syncthreads();
+    int run = wsum[wid] + inc - tot;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int i = 4 * t + q;
+        if (i < nbins) {
+            cnt[i] = run;
+            w.bin_start[i] = run;
+        }
+        run += v[q];
+    }
+    if (t == 0) w.bin_start[nbins] = natoms;
+    __syncthreads();
+    if (t < natoms) w.bin_atoms[cnt[bin] + slot] = t;
+}
+
+// A few list-wide values on the device.
 __global__ void k_set_int(int *p, int v) { *p = v; }
 
-// pair_img[P] = M (both totals read on the device, clamped to the capacities)
-__global__ void k_sentinel(const int32_t *img_ptr, const int32_t *pair_ptr, int natoms, int32_t *pair_img, NLWork w) {
-    const int64_t P = pair_ptr[natoms], M = img_ptr[natoms];
-    if (P <= w.cap_pair) pair_img[P] = (int32_t)(M <= w.cap_img ? M : w.cap_img);
-}
-
-__global__ void k_summary(const int32_t *img_ptr, const int32_t *pair_ptr, int natoms, const int *status, int *out) {
-    out[0] = natoms > 0 ? img_ptr[natoms] : 0;
-    out[1] = (natoms > 0 && pair_ptr) ? pair_ptr[natoms] : 0;
-    out[2] = *status;
-}
-
-// After the summary has recorded the true totals: if a capacity was exceeded (or an
-// offset did not fit), empty every image and pair range, so that kernels enqueued
-// behind the list without a host check (a captured step) read nothing out of bounds.
-__global__ void k_clamp(int32_t *img_ptr, int32_t *pair_ptr, int natoms, const int *status) {
+// {images, pairs, status bits}, and then, if a capacity was exceeded (or an offset did not
+// fit), every image and pair range emptied, so that kernels enqueued behind the list without
+// a host check (a captured step) read nothing out of bounds.  The thread of the last entry
+// takes the totals before it empties its own entry.
+__global__ void k_summary(int32_t *img_ptr, int32_t *pair_ptr, int natoms, const int *status, int *out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > natoms || !(*status & (1 << SO4_ERR_CAPACITY))) return;
+    if (i > natoms) return;
+    const int bits = *status;
+    if (i == natoms) {
+        out[0] = natoms > 0 ? img_ptr[natoms] : 0;
+        out[1] = (natoms > 0 && pair_ptr) ? pair_ptr[natoms] : 0;
+        out[2] = bits;
+    }
+    if (!(bits & (1 << SO4_ERR_CAPACITY))) return;
     img_ptr[i] = 0;
     if (pair_ptr) pair_ptr[i] = 0;
 }
 
-// The range form of k_clamp: after a range's sort, if any capacity was exceeded so far,
-// empty the range's image ranges (img_ptr[a0 .. a1]) before work on them is enqueued.
+// The emptying for a range: after a range's sort, if any capacity was exceeded so far, empty
+// the range's image ranges (img_ptr[a0 .. a1]) before work on them is enqueued.
 __global__ void k_clamp_range(int32_t *img_ptr, int a0, int a1, const int *status) {
     const int i = a0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (i > a1 || !(*(volatile const int *)status & (1 << SO4_ERR_CAPACITY))) return;
@@ -229,112 +293,139 @@ __global__ void k_clamp_range(int32_t *img_ptr, int a0, int a1, const int *statu
 // |r| < rcut - delta surely in, and only the band in between is decided by the
 // exact FP64 test, so the accepted set is exactly the FP64 one while FP64 work
 // (1/64 of the FP32 rate on this GPU) is almost never issued.
-template <int MODE>
-__global__ void k_scan_images(const so4_geom *geom, const double *pos, const int *astruct, int natoms,
-                              double rcut, const int32_t *img_ptr, NLWork w, int a0 = 0) {
+// PARTS warps share a centre, each walking every PARTS-th atom of a bin: the walk is a chain of
+// dependent loads, so while the centres' warps leave the chip half empty (2,432 centres are 64
+// warps on each of 152 SMs at four per centre) shorter chains are faster (64 atoms, bins of
+// eight: 9.2 -> 6.0 us).
+template <int MODE, int PARTS>
+__global__ void __launch_bounds__(256) k_scan_images(const so4_geom *geom, const double *pos, const int *astruct,
+                                                     int natoms, double rcut, const int32_t *img_ptr, NLWork w,
+                                                     int a0 = 0) {
     // centres a0 .. natoms - 1 (a range of the list when a0 > 0)
     __shared__ int s_cnt[8];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int a = a0 + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (MODE >= 1 && lane == 0) s_cnt[wib] = 0;
-    __syncwarp();
-    if (a >= natoms) return;
-    const so4_geom &g = geom[astruct[a]];
-    const double pi[3] = {pos[3 * a], pos[3 * a + 1], pos[3 * a + 2]};
-    const float4 pi32 = w.pos32[a];
-    float c32[9], amax = 0.f;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        c32[q] = (float)g.cell[q];
-        amax = fmaxf(amax, fabsf(c32[q]));
-    }
-    const float rc32 = (float)rcut;
-    const float pimag = fmaxf(fabsf(pi32.x), fmaxf(fabsf(pi32.y), fabsf(pi32.z)));
-    const int lb = w.atom_bin[a] - g.bin_base;
-    const int bi[3] = {lb / (g.nbin[1] * g.nbin[2]), (lb / g.nbin[2]) % g.nbin[1], lb % g.nbin[2]};
-    const int4 si = w.atom_shift[a];
-    const int n1 = 2 * g.mshift[1] + 1, n2 = 2 * g.mshift[2] + 1;
-    const int nq = (2 * g.mshift[0] + 1) * n1 * n2;
-    const int64_t base = (MODE == 1) ? (int64_t)img_ptr[a] : ((MODE == 2) ? (int64_t)a * w.slot_cap : 0);
     int mine = 0;
-    for (int q = lane; q < nq; q += 32) {
-        const int d[3] = {q / (n1 * n2) - g.mshift[0], (q / n2) % n1 - g.mshift[1], q % n2 - g.mshift[2]};
-        int tb[3], img[3];
+    const int wc = wib / PARTS, part = wib - wc * PARTS;  // centre of the CTA, the warp's part of it
+    const int a = a0 + (int)blockIdx.x * (8 / PARTS) + wc;
+    if (part == 0 && lane == 0) s_cnt[wc] = 0;
+    if (PARTS > 1) __syncthreads();
+    else __syncwarp();
+    if (PARTS == 1 && a >= natoms) return;
+    if (a < natoms) {
+        const so4_geom &g = geom[astruct[a]];
+        const double pi[3] = {pos[3 * a], pos[3 * a + 1], pos[3 * a + 2]};
+        const float4 pi32 = w.pos32[a];
+        float c32[9], amax = 0.f;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            // the wrapped bin and the image floor(t / nb), by whole periods: t lies within
-            // mshift of [0, nb), so one step at most unless the cell is thinner than rcut
-            const int nb = g.nbin[k];
-            int wk = bi[k] + d[k], im = 0;
-            while (wk < 0) {
-                wk += nb;
-                --im;
-            }
-            while (wk >= nb) {
-                wk -= nb;
-                ++im;
-            }
-            tb[k] = wk;
-            img[k] = im;
+        for (int q = 0; q < 9; ++q) {
+            c32[q] = (float)g.cell[q];
+            amax = fmaxf(amax, fabsf(c32[q]));
         }
-        const int bin = g.bin_base + (tb[0] * g.nbin[1] + tb[1]) * g.nbin[2] + tb[2];
-        // the next candidate's index is read one ahead, so its loads do not wait on it
-        const int s0 = w.bin_start[bin], s1 = w.bin_start[bin + 1];
-        int jn = (s0 < s1) ? w.bin_atoms[s0] : 0;
-        for (int s = s0; s < s1; ++s) {
-            const int j = jn;
-            if (s + 1 < s1) jn = w.bin_atoms[s + 1];
-            const int4 sj = w.atom_shift[j];
-            const int o[3] = {img[0] + sj.x - si.x, img[1] + sj.y - si.y, img[2] + sj.z - si.z};
-            if (j == a && o[0] == 0 && o[1] == 0 && o[2] == 0) continue;
-            // FP32 prefilter
-            const float4 pj32 = w.pos32[j];
-            const float f0 = (float)o[0], f1 = (float)o[1], f2 = (float)o[2];
-            const float rx = (pj32.x + (f0 * c32[0] + f1 * c32[3] + f2 * c32[6])) - pi32.x;
-            const float ry = (pj32.y + (f0 * c32[1] + f1 * c32[4] + f2 * c32[7])) - pi32.y;
-            const float rz = (pj32.z + (f0 * c32[2] + f1 * c32[5] + f2 * c32[8])) - pi32.z;
-            const float mag = pimag + fmaxf(fabsf(pj32.x), fmaxf(fabsf(pj32.y), fabsf(pj32.z))) +
-                              (fabsf(f0) + fabsf(f1) + fabsf(f2)) * amax;
-            const float delta = 2e-6f * mag + 1e-5f;
-            const float d2 = rx * rx + ry * ry + rz * rz;
-            const float hi = rc32 + delta, lo = rc32 - delta;
-            if (d2 > hi * hi) continue;            // surely outside
-            if (!(lo > 0.f && d2 < lo * lo)) {     // within the rounding band: decide in FP64
-                if (!exact_inside(g, pi, pos, j, o[0], o[1], o[2], rcut)) continue;
-            }
-            if (MODE >= 1) {
-                if (abs(o[0]) > OFF_MAX || abs(o[1]) > OFF_MAX || abs(o[2]) > OFF_MAX) {
-                    flag(w.status, SO4_ERR_CAPACITY);
-                    continue;
+        const float rc32 = (float)rcut;
+        const float pimag = fmaxf(fabsf(pi32.x), fmaxf(fabsf(pi32.y), fabsf(pi32.z)));
+        const int lb = w.atom_bin[a] - g.bin_base;
+        const int bi[3] = {lb / (g.nbin[1] * g.nbin[2]), (lb / g.nbin[2]) % g.nbin[1], lb % g.nbin[2]};
+        const int4 si = w.atom_shift[a];
+        const int n1 = 2 * g.mshift[1] + 1, n2 = 2 * g.mshift[2] + 1;
+        const int nq = (2 * g.mshift[0] + 1) * n1 * n2;
+        const int64_t base = (MODE == 1) ? (int64_t)img_ptr[a] : ((MODE == 2) ? (int64_t)a * w.slot_cap : 0);
+        for (int q = lane; q < nq; q += 32) {
+            const int d[3] = {q / (n1 * n2) - g.mshift[0], (q / n2) % n1 - g.mshift[1], q % n2 - g.mshift[2]};
+            int tb[3], img[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                // the wrapped bin and the image floor(t / nb), by whole periods: t lies within
+                // mshift of [0, nb), so one step at most unless the cell is thinner than rcut
+                const int nb = g.nbin[k];
+                int wk = bi[k] + d[k], im = 0;
+                while (wk < 0) {
+                    wk += nb;
+                    --im;
                 }
-                const unsigned long long key = ((unsigned long long)(unsigned)j << 30) |
-                                               ((unsigned long long)(o[0] + OFF_BIAS) << 20) |
-                                               ((unsigned long long)(o[1] + OFF_BIAS) << 10) |
-                                               (unsigned long long)(o[2] + OFF_BIAS);
-                const int slot = atomicAdd(&s_cnt[wib], 1);
-                if (MODE == 1) {
-                    if (base + slot < w.cap_img) w.keys[base + slot] = key;
-                    else flag(w.status, SO4_ERR_CAPACITY);
-                } else if (slot < w.slot_cap) {
-                    w.keys[base + slot] = key;
-                } else {
-                    flag(w.status, SO4_ERR_SLOTS);
-                    flag(w.status, SO4_ERR_CAPACITY);
+                while (wk >= nb) {
+                    wk -= nb;
+                    ++im;
                 }
+                tb[k] = wk;
+                img[k] = im;
             }
-            ++mine;
+            const int bin = g.bin_base + (tb[0] * g.nbin[1] + tb[1]) * g.nbin[2] + tb[2];
+            // the next candidate's index is read one ahead, so its loads do not wait on it
+            const int s0 = w.bin_start[bin] + part, s1 = w.bin_start[bin + 1];
+            int jn = (s0 < s1) ? w.bin_atoms[s0] : 0;
+            for (int s = s0; s < s1; s += PARTS) {
+                const int j = jn;
+                if (s + PARTS < s1) jn = w.bin_atoms[s + PARTS];
+                const int4 sj = w.atom_shift[j];
+                const int o[3] = {img[0] + sj.x - si.x, img[1] + sj.y - si.y, img[2] + sj.z - si.z};
+                if (j == a && o[0] == 0 && o[1] == 0 && o[2] == 0) continue;
+                // FP32 prefilter
+                const float4 pj32 = w.pos32[j];
+                const float f0 = (float)o[0], f1 = (float)o[1], f2 = (float)o[2];
+                const float rx = (pj32.x + (f0 * c32[0] + f1 * c32[3] + f2 * c32[6])) - pi32.x;
+                const float ry = (pj32.y + (f0 * c32[1] + f1 * c32[4] + f2 * c32[7])) - pi32.y;
+                const float rz = (pj32.z + (f0 * c32[2] + f1 * c32[5] + f2 * c32[8])) - pi32.z;
+                const float mag = pimag + fmaxf(fabsf(pj32.x), fmaxf(fabsf(pj32.y), fabsf(pj32.z))) +
+                                  (fabsf(f0) + fabsf(f1) + fabsf(f2)) * amax;
+                const float delta = 2e-6f * mag + 1e-5f;
+                const float d2 = rx * rx + ry * ry + rz * rz;
+                const float hi = rc32 + delta, lo = rc32 - delta;
+                if (d2 > hi * hi) continue;            // surely outside
+                if (!(lo > 0.f && d2 < lo * lo)) {     // within the rounding band: decide in FP64
+                    if (!exact_inside(g, pi, pos, j, o[0], o[1], o[2], rcut)) continue;
+                }
+                if (MODE >= 1) {
+                    if (abs(o[0]) > OFF_MAX || abs(o[1]) > OFF_MAX || abs(o[2]) > OFF_MAX) {
+                        flag(w.status, SO4_ERR_CAPACITY);
+                        continue;
+                    }
+                    const unsigned long long key = ((unsigned long long)(unsigned)j << 30) |
+                                                   ((unsigned long long)(o[0] + OFF_BIAS) << 20) |
+                                                   ((unsigned long long)(o[1] + OFF_BIAS) << 10) |
+                                                   (unsigned long long)(o[2] + OFF_BIAS);
+                    const int slot = atomicAdd(&s_cnt[wc], 1);
+                    if (MODE == 1) {
+                        if (base + slot < w.cap_img) w.keys[base + slot] = key;
+                        else flag(w.status, SO4_ERR_CAPACITY);
+                    } else if (slot < w.slot_cap) {
+                        w.keys[base + slot] = key;
+                    } else {
+                        flag(w.status, SO4_ERR_SLOTS);
+                        flag(w.status, SO4_ERR_CAPACITY);
+                    }
+                }
+                ++mine;
+            }
+        }
+        if (MODE == 0 || MODE == 2) {
+            int tot = mine;
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
+            // with several warps their sums go through s_cnt (MODE 0) or are its key count (MODE 2,
+            // where a key of an offset out of range is not counted: its status bit empties the list)
+            if (PARTS > 1 && MODE == 0 && lane == 0) atomicAdd(&s_cnt[wc], tot);
+            mine = tot;
         }
     }
-    if (MODE == 0 || MODE == 2) {
-        int tot = mine;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
-        if (lane == 0) {
-            w.cnt[a] = tot;
-            if (tot == 0) flag(w.status, SO4_ERR_NO_NEIGHBOR);
-            if (MODE == 2) atomicMax(w.status + 8, tot);
-        }
+    if (PARTS > 1) __syncthreads();
+    if ((MODE == 0 || MODE == 2) && a < natoms && part == 0 && lane == 0) {
+        const int tot = (PARTS > 1) ? s_cnt[wc] : mine;
+        w.cnt[a] = tot;
+        if (tot == 0) flag(w.status, SO4_ERR_NO_NEIGHBOR);
+        if (MODE == 2) atomicMax(w.status + 8, tot);
     }
+}
+
+// k_scan_images over the centres [a0, a1)
+template <int MODE>
+void launch_scan(const so4_geom *geom, const double *pos, const int *astruct, double rcut, const int32_t *img_ptr,
+                 const NLWork &w, int a0, int a1, cudaStream_t st) {
+    const int n = a1 - a0;
+    if (n <= 2432)
+        k_scan_images<MODE, 4><<<(n + 1) / 2, 256, 0, st>>>(geom, pos, astruct, a1, rcut, img_ptr, w, a0);
+    else
+        k_scan_images<MODE, 1><<<(n + 7) / 8, 256, 0, st>>>(geom, pos, astruct, a1, rcut, img_ptr, w, a0);
+    so4_count_launch();
 }
 
 // One warp per centre: rank-sort the keys, write the sorted images and count pairs.
@@ -368,10 +459,30 @@ __global__ void k_sort(const so4_geom *geom, const double *pos, const int *astru
         zneg[c] = signbit(g.cell[c]) && signbit(g.cell[3 + c]) && signbit(g.cell[6 + c]);
     // keys of this atom: compact at [p0, p1), or in its own slots
     const unsigned long long *kk = w.keys + ((w.slot_cap > 0) ? (int64_t)a * w.slot_cap - p0 : 0);
+    // up to 64 keys are ranked from registers (lane l holds keys l and 32 + l): a shuffle per
+    // comparison instead of a load
+    const int nk = p1 - p0;
+    unsigned long long kreg[2] = {0, 0};
+    int rreg[2] = {0, 0};
+    if (nk <= 64) {
+        if (lane < nk) kreg[0] = kk[p0 + lane];
+        if (lane + 32 < nk) kreg[1] = kk[p0 + lane + 32];
+        for (int p = 0; p < nk; ++p) {
+            const unsigned long long kp = __shfl_sync(0xffffffffu, (p < 32) ? kreg[0] : kreg[1], p & 31);
+            rreg[0] += (kp < kreg[0]) ? 1 : 0;
+            rreg[1] += (kp < kreg[1]) ? 1 : 0;
+        }
+    }
     for (int q = p0 + lane; q < p1; q += 32) {
-        const unsigned long long kq = kk[q];
+        unsigned long long kq;
         int rank = 0;
-        for (int p = p0; p < p1; ++p) rank += (kk[p] < kq) ? 1 : 0;
+        if (nk <= 64) {
+            kq = (q < p0 + 32) ? kreg[0] : kreg[1];
+            rank = (q < p0 + 32) ? rreg[0] : rreg[1];
+        } else {
+            kq = kk[q];
+            for (int p = p0; p < p1; ++p) rank += (kk[p] < kq) ? 1 : 0;
+        }
         const int dst = p0 + rank;
         const int j = (int)(kq >> 30);
         const int o0 = (int)((kq >> 20) & 1023) - OFF_BIAS;
@@ -413,44 +524,58 @@ __global__ void k_sort(const so4_geom *geom, const double *pos, const int *astru
     if (lane == 0) w.cnt[a] = uniq + (self ? 0 : 1);
 }
 
-// One thread per centre: emit its pairs in (sorted j, with (i,i) forced) order.
-__global__ void k_pairs(const so4_geom *geom, const int *astruct, int natoms, const int32_t *img_ptr,
-                        const int32_t *img_j, const int32_t *pair_ptr, int64_t *seq, int32_t *pair_img,
-                        int32_t *nsite, int32_t *img_pair, NLWork w) {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per centre: its pairs in (sorted j, with (i,i) forced) order, lane = image; a centre's
+// pairs are the distinct j of its sorted images, each at its first image.  The last centre's
+// warp also writes pair_img[P] = M (clamped to the capacities).  (A thread per centre walking
+// its images took 13.2 us at 1,000 atoms.)
+__global__ void __launch_bounds__(256) k_pairs(const so4_geom *geom, const int *astruct, int natoms,
+                                               const int32_t *img_ptr, const int32_t *img_j, const int32_t *pair_ptr,
+                                               int64_t *seq, int32_t *pair_img, int32_t *nsite, int32_t *img_pair,
+                                               NLWork w) {
+    const int lane = threadIdx.x & 31;
+    const int a = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (a >= natoms) return;
-    if (img_ptr[a + 1] > w.cap_img || pair_ptr[a + 1] > w.cap_pair) {
-        flag(w.status, SO4_ERR_CAPACITY);
+    const int m0 = img_ptr[a], m1 = img_ptr[a + 1], pp = pair_ptr[a];
+    if (a == natoms - 1 && lane == 0) {
+        const int64_t P = pair_ptr[natoms], M = m1;
+        if (P <= w.cap_pair) pair_img[P] = (int32_t)(M <= w.cap_img ? M : w.cap_img);
+    }
+    if (m1 > w.cap_img || pair_ptr[a + 1] > w.cap_pair) {
+        if (lane == 0) flag(w.status, SO4_ERR_CAPACITY);
         return;
     }
     const int base = geom[astruct[a]].atom_base;
-    int p = pair_ptr[a];
-    int m = img_ptr[a];
-    const int me = img_ptr[a + 1];
-    bool self_done = false;
-    while (m < me || !self_done) {
-        const int j = (m < me) ? img_j[m] : 0x7fffffff;
-        if (!self_done && a < j) {
-            seq[2 * p] = a - base;
-            seq[2 * p + 1] = a - base;
+    bool self = false;  // an image of the centre itself
+    int below = 0;      // images of j < a
+    for (int m = m0 + lane; m < m1; m += 32) {
+        const int j = img_j[m];
+        self |= j == a;
+        below += (j < a) ? 1 : 0;
+    }
+    self = __any_sync(0xffffffffu, self);
+    below = __reduce_add_sync(0xffffffffu, below);
+    int seen = 0, before = 0;  // distinct j so far, and those below a
+    for (int mb = m0; mb < m1; mb += 32) {
+        const int m = mb + lane;
+        const int j = (m < m1) ? img_j[m] : 0x7fffffff;
+        const bool fresh = m < m1 && (m == m0 || img_j[m - 1] != j);
+        const unsigned fm = __ballot_sync(0xffffffffu, fresh);
+        const int p = pp + seen + __popc(fm & (0xffffffffu >> (31 - lane))) - 1 + ((!self && j > a) ? 1 : 0);
+        if (m < m1) img_pair[m] = p;
+        if (fresh) {
+            seq[2 * (int64_t)p] = a - base;
+            seq[2 * (int64_t)p + 1] = j - base;
             pair_img[p] = m;
-            nsite[a] = p;
-            ++p;
-            self_done = true;
-            continue;
+            if (j == a) nsite[a] = p;
         }
-        seq[2 * p] = a - base;
-        seq[2 * p + 1] = j - base;
-        pair_img[p] = m;
-        if (j == a) {
-            nsite[a] = p;
-            self_done = true;
-        }
-        while (m < me && img_j[m] == j) {
-            img_pair[m] = p;
-            ++m;
-        }
-        ++p;
+        before += __popc(__ballot_sync(0xffffffffu, fresh && j < a));
+        seen += __popc(fm);
+    }
+    if (!self && lane == 0) {
+        const int p = pp + before;
+        seq[2 * (int64_t)p] = seq[2 * (int64_t)p + 1] = a - base;
+        pair_img[p] = m0 + below;
+        nsite[a] = p;
     }
 }
 
@@ -590,6 +715,23 @@ extern "C" size_t so4_nl_workspace_size(int natoms, int nbins_total, int64_t nim
     return carve(w, nullptr, natoms, nbins_total, nimg);
 }
 
+// Header cleared, every atom in its bin.
+static int make_bins(const NLWork &w, const so4_geom *d_geom, int nbins, const double *d_pos, const int *d_astruct,
+                     int natoms, cudaStream_t st) {
+    if (natoms <= BIN_ATOMS && nbins <= BIN_BINS) {
+        k_bin_small<<<1, 1024, 0, st>>>(d_geom, d_pos, d_astruct, natoms, nbins, w);
+        so4_count_launch();
+        return SO4_OK;
+    }
+    SO4_CUDA_TRY(cudaMemsetAsync(w.status, 0, w.clear, st));
+    const int tb = 256;
+    k_bin<<<(natoms + tb - 1) / tb, tb, 0, st>>>(d_geom, d_pos, d_astruct, natoms, w);
+    k_scan<<<1, 1024, 0, st>>>(w.bin_cnt, w.bin_start, nbins);
+    k_bin_fill<<<(natoms + tb - 1) / tb, tb, 0, st>>>(d_astruct, natoms, w);
+    so4_count_launch(3);
+    return SO4_OK;
+}
+
 extern "C" int so4_nl_count(const so4_geom *d_geom, int nstruct, int nbins, const double *d_pos, const int *d_astruct,
                             int natoms, double rcut, int32_t *d_img_ptr, void *d_work, size_t work_bytes,
                             void *stream) {
@@ -601,25 +743,15 @@ extern "C" int so4_nl_count(const so4_geom *d_geom, int nstruct, int nbins, cons
     w.cap_pair = 0;
     w.slot_cap = 0;
     cudaStream_t st = (cudaStream_t)stream;
-    SO4_CUDA_TRY(cudaMemsetAsync(w.status, 0, sizeof(int), st));
     if (natoms == 0) {
+        SO4_CUDA_TRY(cudaMemsetAsync(w.status, 0, sizeof(int), st));
         k_set_int<<<1, 1, 0, st>>>(d_img_ptr, 0);
         so4_count_launch();
         return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
     }
-    SO4_CUDA_TRY(cudaMemsetAsync(w.bin_cnt, 0, sizeof(int) * (nbins + 1), st));
-    SO4_CUDA_TRY(cudaMemsetAsync(w.bin_cur, 0, sizeof(int) * (nbins + 1), st));
-    const int tb = 256;
-    k_bin<<<(natoms + tb - 1) / tb, tb, 0, st>>>(d_geom, d_pos, d_astruct, natoms, w);
-    so4_count_launch();
-    k_scan<<<1, 1024, 0, st>>>(w.bin_cnt, w.bin_start, nbins);
-    so4_count_launch();
-    k_bin_fill<<<(natoms + tb - 1) / tb, tb, 0, st>>>(d_astruct, natoms, w);
-    so4_count_launch();
-    const int warps = 8;
-    k_scan_images<0><<<(natoms + warps - 1) / warps, 32 * warps, 0, st>>>(d_geom, d_pos, d_astruct, natoms, rcut,
-                                                                          nullptr, w);
-    so4_count_launch();
+    const int rc = make_bins(w, d_geom, nbins, d_pos, d_astruct, natoms, st);
+    if (rc) return rc;
+    launch_scan<0>(d_geom, d_pos, d_astruct, rcut, nullptr, w, 0, natoms, st);
     k_scan<<<1, 1024, 0, st>>>(w.cnt, d_img_ptr, natoms);
     so4_count_launch();
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
@@ -645,8 +777,7 @@ extern "C" int so4_nl_fill(const so4_geom *d_geom, int nstruct, int nbins, const
     }
     const int warps = 8;
     const int grid = (natoms + warps - 1) / warps;
-    k_scan_images<1><<<grid, 32 * warps, 0, st>>>(d_geom, d_pos, d_astruct, natoms, rcut, d_img_ptr, w);
-    so4_count_launch();
+    launch_scan<1>(d_geom, d_pos, d_astruct, rcut, d_img_ptr, w, 0, natoms, st);
     k_sort<<<grid, 32 * warps, 0, st>>>(d_geom, d_pos, d_astruct, natoms, d_img_ptr, d_img_j, d_img_off, d_img_r, w);
     so4_count_launch();
     k_scan<<<1, 1024, 0, st>>>(w.cnt, d_pair_ptr, natoms);
@@ -671,17 +802,12 @@ extern "C" int so4_nl_bins(const so4_geom *d_geom, int nstruct, int nbins, const
     int rc = one_pass_work(w, natoms, nbins, slot_cap, d_work, work_bytes);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    SO4_CUDA_TRY(cudaMemsetAsync(w.status, 0, 9 * sizeof(int), st));  // status, summary, largest count
-    if (natoms == 0) return SO4_OK;
-    SO4_CUDA_TRY(cudaMemsetAsync(w.bin_cnt, 0, sizeof(int) * (nbins + 1), st));
-    SO4_CUDA_TRY(cudaMemsetAsync(w.bin_cur, 0, sizeof(int) * (nbins + 1), st));
-    const int tb = 256;
-    k_bin<<<(natoms + tb - 1) / tb, tb, 0, st>>>(d_geom, d_pos, d_astruct, natoms, w);
-    so4_count_launch();
-    k_scan<<<1, 1024, 0, st>>>(w.bin_cnt, w.bin_start, nbins);
-    so4_count_launch();
-    k_bin_fill<<<(natoms + tb - 1) / tb, tb, 0, st>>>(d_astruct, natoms, w);
-    so4_count_launch();
+    if (natoms == 0) {
+        SO4_CUDA_TRY(cudaMemsetAsync(w.status, 0, 9 * sizeof(int), st));  // status, summary, largest count
+        return SO4_OK;
+    }
+    rc = make_bins(w, d_geom, nbins, d_pos, d_astruct, natoms, st);
+    if (rc) return rc;
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
 }
 
@@ -694,10 +820,7 @@ extern "C" int so4_nl_count_keys_range(const so4_geom *d_geom, int nstruct, int 
     int rc = one_pass_work(w, natoms, nbins, slot_cap, d_work, work_bytes);
     if (rc) return rc;
     if (a1 == a0) return SO4_OK;
-    const int warps = 8;
-    k_scan_images<2><<<(a1 - a0 + warps - 1) / warps, 32 * warps, 0, (cudaStream_t)stream>>>(
-        d_geom, d_pos, d_astruct, a1, rcut, nullptr, w, a0);
-    so4_count_launch();
+    launch_scan<2>(d_geom, d_pos, d_astruct, rcut, nullptr, w, a0, a1, (cudaStream_t)stream);
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
 }
 
@@ -769,16 +892,20 @@ extern "C" int so4_nl_sort(const so4_geom *d_geom, int nstruct, int nbins, const
     w.slot_cap = slot_cap;
     cudaStream_t st = (cudaStream_t)stream;
     if (natoms == 0) {
-        k_set_int<<<1, 1, 0, st>>>(d_pair_ptr, 0);
-        so4_count_launch();
+        if (d_pair_ptr) {
+            k_set_int<<<1, 1, 0, st>>>(d_pair_ptr, 0);
+            so4_count_launch();
+        }
         return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
     }
     const int warps = 8;
     const int grid = (natoms + warps - 1) / warps;
     k_sort<<<grid, 32 * warps, 0, st>>>(d_geom, d_pos, d_astruct, natoms, d_img_ptr, d_img_j, d_img_off, d_img_r, w);
     so4_count_launch();
-    k_scan<<<1, 1024, 0, st>>>(w.cnt, d_pair_ptr, natoms);
-    so4_count_launch();
+    if (d_pair_ptr) {
+        k_scan<<<1, 1024, 0, st>>>(w.cnt, d_pair_ptr, natoms);
+        so4_count_launch();
+    }
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
 }
 
@@ -804,10 +931,7 @@ extern "C" int so4_nl_pairs(const so4_geom *d_geom, int nstruct, const int *d_as
     }
     const bool pairs = d_seq && d_pair_img && d_nsite && d_img_pair;
     if (pairs) {
-        k_sentinel<<<1, 1, 0, st>>>(d_img_ptr, d_pair_ptr, natoms, d_pair_img, w);
-        so4_count_launch();
-        const int tb = 128;
-        k_pairs<<<(natoms + tb - 1) / tb, tb, 0, st>>>(d_geom, d_astruct, natoms, d_img_ptr, d_img_j, d_pair_ptr,
+        k_pairs<<<(natoms + 7) / 8, 256, 0, st>>>(d_geom, d_astruct, natoms, d_img_ptr, d_img_j, d_pair_ptr,
                                                        d_seq, d_pair_img, d_nsite, d_img_pair, w);
         so4_count_launch();
     }
@@ -835,10 +959,8 @@ extern "C" int so4_nl_summary(const int32_t *d_img_ptr, const int32_t *d_pair_pt
     if (!d_work || work_bytes < SO4_WS_HEADER || natoms < 0) return SO4_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
     int *dev = (int *)d_work + 4;  // header scratch after the status word
-    k_summary<<<1, 1, 0, st>>>(d_img_ptr, d_pair_ptr, natoms, (const int *)d_work, dev);
-    so4_count_launch();
-    k_clamp<<<(natoms + 256) / 256, 256, 0, st>>>((int32_t *)d_img_ptr, (int32_t *)d_pair_ptr, natoms,
-                                                  (const int *)d_work);
+    k_summary<<<(natoms + 256) / 256, 256, 0, st>>>((int32_t *)d_img_ptr, (int32_t *)d_pair_ptr, natoms,
+                                                    (const int *)d_work, dev);
     so4_count_launch();
     if (!h_summary) return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
     SO4_CUDA_TRY(cudaMemcpyAsync(h_summary, dev, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -225,19 +225,21 @@ class NeighborBuffers:
         return self.ws[32:36].view(torch.int32)
 
 
-def enqueue_neighbors(lay: Layout, pos, bufs: NeighborBuffers, summary=None, lite=False):
+def enqueue_neighbors(lay: Layout, pos, bufs: NeighborBuffers, summary=None, lite=False, count_pairs=True):
     """Launch the three neighbour-list passes for positions pos (N,3) f64 on the device
     into bufs, and the summary; with summary (a ctypes int[3]) the call waits and
     fills it, else nothing synchronises (the summary stays on the device).  lite: skip
-    the pair arrays (seq, pair_img, nsite, img_pair), keeping what the adjoint reads."""
+    the pair arrays (seq, pair_img, nsite, img_pair), keeping what the adjoint reads;
+    count_pairs False (with lite, in the slot mode): their number too (0 in the summary)."""
     L, st, N, S = lib(), _stream(), lay.natoms, lay.nstruct
     b = bufs
+    pair_ptr = b.pair_ptr if count_pairs else None
     if b.slot_cap > 0:
         check(L.so4_nl_count_keys(_ptr(lay.geom), S, lay.nbins, _ptr(pos), _ptr(lay.atom_struct), N, lay.rcut,
                                   b.slot_cap, _ptr(b.img_ptr), _ptr(b.ws), b.ws.numel(), st), "so4_nl_count_keys")
         check(L.so4_nl_sort(_ptr(lay.geom), S, lay.nbins, _ptr(pos), _ptr(lay.atom_struct), N, _ptr(b.img_ptr),
-                            b.cap_m, b.slot_cap, _ptr(b.img_j), _ptr(b.img_off), _ptr(b.img_r), _ptr(b.pair_ptr),
-                            _ptr(b.ws), b.ws.numel(), st), "so4_nl_sort")
+                            b.cap_m, b.slot_cap, _ptr(b.img_j), _ptr(b.img_off), _ptr(b.img_r),
+                            _ptr(pair_ptr), _ptr(b.ws), b.ws.numel(), st), "so4_nl_sort")
     else:
         check(L.so4_nl_count(_ptr(lay.geom), S, lay.nbins, _ptr(pos), _ptr(lay.atom_struct), N, lay.rcut,
                              _ptr(b.img_ptr), _ptr(b.ws), b.ws.numel(), st), "so4_nl_count")
@@ -250,8 +252,8 @@ def enqueue_neighbors(lay: Layout, pos, bufs: NeighborBuffers, summary=None, lit
                          _ptr(b.pair_img if pairs else None), _ptr(b.nsite if pairs else None),
                          _ptr(b.img_pair if pairs else None), _ptr(b.img_rev), _ptr(b.ws), b.ws.numel(), st),
           "so4_nl_pairs")
-    check(L.so4_nl_summary(_ptr(b.img_ptr), _ptr(b.pair_ptr), N, _ptr(b.ws), b.ws.numel(), st, summary),
-          "so4_nl_summary")
+    check(L.so4_nl_summary(_ptr(b.img_ptr), _ptr(pair_ptr), N, _ptr(b.ws), b.ws.numel(), st,
+                           summary), "so4_nl_summary")
 
 
 def check_summary(M, P, bits, cap_m=None, cap_p=None):
@@ -491,6 +493,14 @@ def gather(nb: Neighbors, g, eatom=None):
                                    _ptr(nb.img_r), _ptr(g), _ptr(eatom), _ptr(part), _ptr(forces), _ptr(virial),
                                    _ptr(energy), _stream()), "so4_adjoint_gather")
     return forces[:N], virial[: nb.nstruct], (energy[: nb.nstruct] if energy is not None else None)
+
+
+def virial_stress(virial, vol):
+    """Stress (S, 6) f64 in GPa, xx yy zz xy xz yz, of virials (S, 3, 3) and volumes (S,) on the device."""
+    S = virial.shape[0]
+    out = torch.empty((S, 6), dtype=torch.float64, device=virial.device)
+    check(lib().so4_virial_stress(S, _ptr(virial), _ptr(vol), _ptr(out), _stream()), "so4_virial_stress")
+    return out
 
 
 def adjoint32_staged(tab, prm, nb: Neighbors, w_nb, utot, beta, mark=None, first=0):
