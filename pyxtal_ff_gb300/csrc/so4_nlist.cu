@@ -199,9 +199,10 @@ __global__ void __launch_bounds__(1024) k_scan(const int *in, int *out, int n, i
 // The bins of a small list (natoms <= BIN_ATOMS, nbins <= BIN_BINS) by one CTA: header cleared,
 // atoms binned (thread = atom), bin starts scanned and filled, in one launch instead of a
 // clear and three kernels.  Its FP64 work (about 30 operations per atom, 2 per cycle and SM)
-// stays below the latencies that it saves: 64 atoms 5.1 us instead of 9.9, 1,000 atoms 12.0
-// instead of 13.1 (sums of the kernels; each launch also has a gap of about 1 us).
-constexpr int BIN_ATOMS = 1024, BIN_BINS = 4096;
+// stays below the latencies that it saves: 216 atoms 5.0 us instead of 8.7 (sums of the kernels;
+// each launch also has a gap of about 1 us), 512 atoms 8.3 instead of 9.2; not at 1,000 atoms,
+// 14.2 instead of 9.2.
+constexpr int BIN_ATOMS = 640, BIN_BINS = 4096;
 __global__ void __launch_bounds__(1024) k_bin_small(const so4_geom *geom, const double *pos, const int *astruct,
                                                     int natoms, int nbins, NLWork w) {
     __shared__ int cnt[BIN_BINS], wsum[32];
@@ -294,9 +295,10 @@ __global__ void k_clamp_range(int32_t *img_ptr, int a0, int a1, const int *statu
 // exact FP64 test, so the accepted set is exactly the FP64 one while FP64 work
 // (1/64 of the FP32 rate on this GPU) is almost never issued.
 // PARTS warps share a centre, each walking every PARTS-th atom of a bin: the walk is a chain of
-// dependent loads, so while the centres' warps leave the chip half empty (2,432 centres are 64
-// warps on each of 152 SMs at four per centre) shorter chains are faster (64 atoms, bins of
-// eight: 9.2 -> 6.0 us).
+// dependent loads, so while the centres' warps leave the chip half empty (1,216 centres are 32
+// warps on each of 152 SMs at four per centre) shorter chains are faster: the two passes over
+// 216 atoms 10.7 us instead of 17.1, 1,000 atoms 14.7 instead of 18.0, but 1,728 atoms 23.0
+// instead of 18.9.
 template <int MODE, int PARTS>
 __global__ void __launch_bounds__(256) k_scan_images(const so4_geom *geom, const double *pos, const int *astruct,
                                                      int natoms, double rcut, const int32_t *img_ptr, NLWork w,
@@ -421,7 +423,7 @@ template <int MODE>
 void launch_scan(const so4_geom *geom, const double *pos, const int *astruct, double rcut, const int32_t *img_ptr,
                  const NLWork &w, int a0, int a1, cudaStream_t st) {
     const int n = a1 - a0;
-    if (n <= 2432)
+    if (n <= 1216)
         k_scan_images<MODE, 4><<<(n + 1) / 2, 256, 0, st>>>(geom, pos, astruct, a1, rcut, img_ptr, w, a0);
     else
         k_scan_images<MODE, 1><<<(n + 7) / 8, 256, 0, st>>>(geom, pos, astruct, a1, rcut, img_ptr, w, a0);

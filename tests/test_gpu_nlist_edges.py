@@ -1,5 +1,5 @@
-"""The neighbour list where its kernels change: one CTA or several for the bins (1,024 atoms,
-4,096 bins), four warps or one per centre (2,432 centres), keys ranked from registers or from
+"""The neighbour list where its kernels change: one CTA or several for the bins (640 atoms,
+4,096 bins), four warps or one per centre (1,216 centres), keys ranked from registers or from
 memory (64 images), pairs of a centre with more than 32 images, with and without images of its
 own.  Bit for bit the oracle's list: no tolerance.
 """
@@ -20,10 +20,10 @@ def _si(*n):
 
 
 CASES = {
-    "1024 atoms": ([_si(8, 4, 4)], 3.0),
-    "1032 atoms": ([_si(43, 3, 1)], 3.0),
-    "2432 atoms": ([_si(19, 16, 1)], 3.0),
-    "2440 atoms": ([_si(61, 5, 1)], 3.0),
+    "640 atoms": ([_si(5, 4, 4)], 3.0),
+    "648 atoms": ([_si(9, 3, 3)], 3.0),
+    "1216 atoms": ([_si(19, 8, 1)], 3.0),
+    "1224 atoms": ([_si(17, 9, 1)], 3.0),
     "more than 4096 bins": ([S.Atoms([14] * 5, np.random.default_rng(72).uniform(0, 90, (5, 3)), 90 * np.eye(3)),
                              _si(1, 1, 1)], 5.2),
     "64 images and more": ([_si(1, 1, 1), S.Atoms([14], [[0.1, 0.2, 0.3]], 2.8 * np.eye(3)), _si(2, 1, 1)], 6.9),
