@@ -448,21 +448,41 @@ void so4_count_launch(int n = 1);
 int so4_pdl_on();
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Barrier over the CTAs of a cluster; what their threads wrote before it, to global memory
+// too, is visible to all of them after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// cluster: CTAs of a cluster along x (1: none)
 template <typename... KArgs, typename... Args>
-int so4_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+int so4_launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t st,
+                       Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (so4_pdl_on()) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster;
+        at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = at;
-    cfg.numAttrs = so4_pdl_on() ? 1 : 0;
+    cfg.numAttrs = n;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
     so4_count_launch();
     return e == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
+}
+template <typename... KArgs, typename... Args>
+int so4_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+    return so4_launch_cluster(kern, grid, block, smem, 1, st, std::forward<Args>(args)...);
 }
 // Raise a kernel's dynamic shared-memory limit to at least smem bytes on the current
 // device.  The attribute is set only when the limit grows, so launches after the

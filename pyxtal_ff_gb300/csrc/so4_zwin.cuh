@@ -66,8 +66,8 @@ __device__ __forceinline__ void zw_load_utot(const float2 *__restrict__ utot, co
 // scratch sc[q * natoms + a0 + l], for every k < ncomp and every l < NA with a0 + l <
 // natoms, handed to f(k, l, sum, pre(k, l)).  The CTA (NT threads, NA atoms) copies its
 // nslot x NA values into shared memory (stage: nslot x (NA + 1) floats) with independent
-// loads, issued together with pre() of the thread's first NPRE (k, l) pairs, then sums from
-// there in slot order.
+// loads (from L2: other CTAs of a cluster may have written them), issued together with pre() of
+// the thread's first NPRE (k, l) pairs, then sums from there in slot order.
 constexpr int ZW_SLD = 24;
 template <int NPRE, int NA = 32, int NT = ZW_THREADS, typename P, typename F>
 __device__ __forceinline__ void zw_slot_sums(const float *sc, const int *__restrict__ pos, int ncomp, int nslot,
@@ -85,7 +85,7 @@ __device__ __forceinline__ void zw_slot_sums(const float *sc, const int *__restr
 #pragma unroll
         for (int r = 0; r < ZW_SLD; ++r) {
             const int i = i0 + r * NT, q = i / NA, l = i % NA;
-            v[r] = (i < NA * nslot && l < nl) ? sc[(size_t)q * natoms + a0 + l] : 0.f;
+            v[r] = (i < NA * nslot && l < nl) ? __ldcg(sc + (size_t)q * natoms + a0 + l) : 0.f;
         }
 #pragma unroll
         for (int r = 0; r < ZW_SLD; ++r) {
@@ -132,7 +132,7 @@ __device__ __forceinline__ void zw_slot_sums_chunked(const float *sc, const int 
 #pragma unroll
             for (int r = 0; r < ZW_SLD; ++r) {
                 const int i = i0 + r * NT, q = i / NA, l = i % NA;
-                v[r] = (i < NA * nq && l < nl) ? sc[(size_t)(q0 + q) * natoms + a0 + l] : 0.f;
+                v[r] = (i < NA * nq && l < nl) ? __ldcg(sc + (size_t)(q0 + q) * natoms + a0 + l) : 0.f;
             }
 #pragma unroll
             for (int r = 0; r < ZW_SLD; ++r) {
