@@ -65,10 +65,10 @@ def compute_descriptor(function, structure):
     return _descriptor_object(function).calculate(structure, stress_per_atom=True)
 
 
-def _symbols(atoms):
-    if hasattr(atoms, "get_chemical_symbols"):
-        return list(atoms.get_chemical_symbols())
-    return list(atoms.symbols)
+def _element_order(symbols, elements):
+    """The atoms element after element, as the networks' energies are stored."""
+    symbols = np.asarray(symbols)
+    return np.concatenate([np.nonzero(symbols == e)[0] for e in elements])
 
 
 class PyXtalFFCalculator:
@@ -85,7 +85,7 @@ class PyXtalFFCalculator:
         self.atoms = None
         self._atoms_obj = None
         self._calc = None
-        self._step, self._step_key, self._last_key = None, None, None
+        self._step, self._step_key, self._last_key, self._order = None, None, None, None
 
     def _ff(self):
         ff = self.parameters["ff"]
@@ -105,7 +105,9 @@ class PyXtalFFCalculator:
         return any(a.shape != b.shape or not np.array_equal(a, b) for a, b in zip(self._key(atoms), self.atoms))
 
     def _adjoint(self, atoms, ff):
+        from . import engine
         from .calculator import EV_A3_TO_GPA, Batch, SO4Calculator
+        from .structures import as_arrays
         if ff.model.unit == "Ha":
             raise NotImplementedError("route='adjoint' supports unit 'eV'")
         f = ff._descriptors
@@ -117,32 +119,46 @@ class PyXtalFFCalculator:
             self._calc = SO4Calculator(lmax=p["lmax"], rcut=f["Rc"], kind=kind, weights=f.get("weights"),
                                        rfac0=p.get("rfac", 0.99363), cutoff_function=f["cutoff"],
                                        normalize_U=p.get("normalize_U", False))
-        batch = Batch([atoms])
         # an MD or relaxation loop moves only the positions: from the second structure of one
         # layout (cell, pbc, species, model) on, the step is one CUDA-graph replay
         # (SO4Calculator.capture), bit for bit the uncaptured compute()
-        key = (batch.cells.tobytes(), np.asarray(batch.pbc).tobytes(), np.asarray(atoms.numbers).tobytes(),
-               id(ff.model), tuple(id(ff.model.models[e]) for e in ff.model.elements))
+        positions, cell, pbc, numbers, symbols = as_arrays(atoms)
+        key = (cell.tobytes(), pbc.tobytes(), numbers.tobytes(), symbols, id(ff.model), tuple(ff.model.elements),
+               tuple(id(ff.model.models[e]) for e in ff.model.elements))
         if self._step is not None and self._step_key != key:
             self._step = None
         if self._step is None and self._last_key == key:
+            batch = Batch([atoms])
             self._step = self._calc.capture(batch, ff.model.energy_model(batch.species_order))
             self._step_key = key
+            self._order = _element_order(symbols, ff.model.elements)
         self._last_key = key
         r = None
         if self._step is not None:
-            r = self._step(batch.positions)
+            r = self._step(positions)
+            order = self._order
             if not self._step.check():  # the neighbour list outgrew the captured buffers
                 self._step, r = None, None
         if r is None:
+            batch = Batch([atoms])
             r = self._calc.compute(batch, ff.model.energy_model(batch.species_order))
-        e_atom = r["energies"].double()
-        symbols = np.asarray(_symbols(atoms))
-        order = np.concatenate([np.nonzero(symbols == e)[0] for e in ff.model.elements])
-        energies = e_atom.cpu().numpy()[order]
-        forces = r["forces"].cpu().numpy()
-        stress = r["stress"][0].cpu().numpy() / EV_A3_TO_GPA * EV2GPA
-        return energies, forces, stress
+            order = _element_order(symbols, ff.model.elements)
+        energies, forces, stress = engine.to_host(r["energies"].double(), r["forces"], r["stress"])
+        return energies[order], forces, stress[0] / EV_A3_TO_GPA * EV2GPA
+
+    def _plain(self, atoms, ff):
+        if type(ff.model).calculate_properties is not NeuralNetworkPotential.calculate_properties:
+            self.desp = compute_descriptor(ff._descriptors, atoms)
+            return ff.model.calculate_properties(self.desp, bforce=True, bstress=True)
+        # the same two calls with the descriptors left on the device between them
+        function = _descriptor_object(ff._descriptors)
+        desp, nb = function._device(atoms, stress_per_atom=True)
+        d = ff.model._device_properties(desp, True, True, pair_ptr=nb.pair_ptr)
+        n = d[0].shape[0]
+        properties = function._to_host(desp, *d)
+        out = ff.model._host_properties(*properties, n=n)
+        self.desp = desp
+        return out
 
     def calculate(self, atoms=None, properties=("energy",), system_changes=None):
         if atoms is None:
@@ -150,9 +166,7 @@ class PyXtalFFCalculator:
         self._atoms_obj = atoms
         ff = self._ff()
         if self.route == "plain":
-            desp = compute_descriptor(ff._descriptors, atoms)
-            energies, forces, stress = ff.model.calculate_properties(desp, bforce=True, bstress=True)
-            self.desp = desp
+            energies, forces, stress = self._plain(atoms, ff)
         else:
             energies, forces, stress = self._adjoint(atoms, ff)
         n = len(atoms.positions)

@@ -164,22 +164,31 @@ class SO4Calculator:
             positions = torch.from_numpy(np.ascontiguousarray(positions, dtype=np.float64))
         return positions.to(self.device, dtype=torch.float64, non_blocking=True).contiguous()
 
+    def _compute_linear(self, nb, model):
+        beta = model.coef.detach()[self._species]
+        need = engine.lib().so4_linear_workspace_size(self.tables.handle, nb.natoms, nb.nimg)
+        if self._ws is None or self._ws.numel() < need:
+            self._ws = torch.empty(int(need * 1.25) + 4096, dtype=torch.uint8, device=self.device)
+        x, forces, virial, energy = engine.adjoint_linear32(self.tables, self.params, nb, self._w_nb, self._w_site, beta,
+                                                            workspace=self._ws)
+        energy = energy + self._counts @ model.bias.detach().double()
+        return dict(energy=energy, forces=forces, virial=virial, stress=engine.virial_stress(virial, self._vol), x=x)
+
     def compute(self, batch: Batch, model, positions=None):
         """Energy (S,) f64, forces (N,3) f64, virial (S,3,3) f64, stress (S,6) GPa and B."""
         self.prepare(batch)
         pos = self._positions(batch, positions)
-        nb = self.neighbors(batch, pos)
         if isinstance(model, LinearModel):
-            # beta = dE/dB does not depend on B: forward and adjoint in one fused pass
-            beta = model.coef.detach()[self._species]
-            need = engine.lib().so4_linear_workspace_size(self.tables.handle, nb.natoms, nb.nimg)
-            if self._ws is None or self._ws.numel() < need:
-                self._ws = torch.empty(int(need * 1.25) + 4096, dtype=torch.uint8, device=self.device)
-            x, forces, virial, energy = engine.adjoint_linear32(self.tables, self.params, nb, self._w_nb,
-                                                                self._w_site, beta, workspace=self._ws)
-            energy = energy + self._counts @ model.bias.detach().double()
-            stress = engine.virial_stress(virial, self._vol)
-            return dict(energy=energy, forces=forces, virial=virial, stress=stress, x=x, neighbors=nb)
+            # beta = dE/dB does not depend on B: forward and adjoint in one fused pass, launched
+            # behind the neighbour list before its counts are read
+            nb, finish = engine.start_neighbors(pos, batch.cells, batch.pbc, batch.atom_ptr, self.rcut, self.device)
+            out = self._compute_linear(nb, model)
+            nb = finish()
+            if nb is None:
+                nb = self.neighbors(batch, pos)
+                out = self._compute_linear(nb, model)
+            return dict(out, neighbors=nb)
+        nb = self.neighbors(batch, pos)
         x, utot = engine.forward32(self.tables, self.params, nb, self._w_nb, self._w_site)
         xg = x.detach().requires_grad_(True)
         with torch.enable_grad():

@@ -106,6 +106,26 @@ class BispectrumBase:
         caller reduces it after calculate() (pyxtal_ff/utilities/__init__.py:226-233):
         one (len(x), nB, 6) Voigt row block per centre, summed on the GPU, so the
         per-pair array never leaves the device."""
+        from .. import engine
+
+        res, _ = self._device(atoms, atom_ids, stress_per_atom)
+        self._to_host(res)
+        self.clear_memory()
+        return res
+
+    @staticmethod
+    def _to_host(res, *more):
+        """The device arrays of _device()'s dict copied to numpy, in place, together with `more`
+        device tensors, which are returned as arrays."""
+        from .. import engine
+        keys = [k for k in ("x", "dxdr", "seq", "rdxdr") if res.get(k) is not None and not isinstance(res[k], np.ndarray)]
+        got = engine.to_host(*[res[k] for k in keys], *more)
+        res.update(zip(keys, got))
+        return got[len(keys):]
+
+    def _device(self, atoms, atom_ids=None, stress_per_atom=False):
+        """calculate()'s dict with its arrays still on the device (but for an rdxdr that no kernel
+        computes), and the neighbour list."""
         import torch
         from .. import engine
         from ..structures import as_arrays
@@ -130,31 +150,28 @@ class BispectrumBase:
         prm = engine.params(twol, self._rcut, self._rfac0(), self._cutoff_function)
         pos_d = torch.from_numpy(pos).to(dev)
         nb = engine.build_neighbors(pos_d, cell[None], pbc[None], [0, n], self._rcut, device=dev)
-        counts = np.diff(nb.img_ptr[: k + 1].cpu().numpy())
-        if k and np.any(counts == 0):
-            # the reference cannot pad an empty neighbour list (SO4.py:274-276 raises
-            # "could not broadcast input array from shape (0,) into shape (0,3)")
-            i = int(np.nonzero(counts == 0)[0][0])
-            raise ValueError("atom %d has no neighbour within rcut=%g" % (i, self._rcut))
-        w_nb, w_site = self._weights(numbers, symbols)
-        w_nb_d = torch.from_numpy(w_nb).to(dev)
-        w_site_d = torch.from_numpy(w_site).to(dev)
+        if k and nb.no_neighbor:
+            counts = np.diff(nb.img_ptr[: k + 1].cpu().numpy())
+            if np.any(counts == 0):
+                # the reference cannot pad an empty neighbour list (SO4.py:274-276 raises
+                # "could not broadcast input array from shape (0,) into shape (0,3)")
+                i = int(np.nonzero(counts == 0)[0][0])
+                raise ValueError("atom %d has no neighbour within rcut=%g" % (i, self._rcut))
+        w_nb_d, w_site_d = torch.from_numpy(np.stack(self._weights(numbers, symbols))).to(dev)
         x, dxdr, rdxdr = engine.plain(tab, prm, nb, pos_d, w_nb_d, w_site_d, precision=0,
                                       want_deriv=self._derivative, want_stress=self._stress)
-        pk = int(nb.pair_ptr[k].item())
-        out_x = x[:k].cpu().numpy()
+        pk = nb.npair if k == n else int(nb.pair_ptr[k].item())
         elements = list(atoms.symbols)
         if self._derivative:
-            res = {"x": out_x, "dxdr": dxdr[:pk].cpu().numpy(), "elements": elements,
-                   "seq": nb.seq[:pk].cpu().numpy()}
+            res = {"x": x[:k], "dxdr": dxdr[:pk], "elements": elements, "seq": nb.seq[:pk]}
             if not self._stress:
                 res["rdxdr"] = None
             elif stress_per_atom:
-                res["rdxdr"] = engine.rdxdr_atom(rdxdr, nb.pair_ptr, k).cpu().numpy()
+                res["rdxdr"] = engine.rdxdr_atom(rdxdr, nb.pair_ptr, k)
             else:
-                res["rdxdr"] = rdxdr[:pk].cpu().numpy()
+                res["rdxdr"] = rdxdr[:pk]
         else:
-            res = {"x": out_x, "dxdr": None, "elements": elements}
+            res = {"x": x[:k], "dxdr": None, "elements": elements}
             # without derivatives the reference never fills bstress (SO4.py:1671-1728),
             # so it returns -0/vol over every pair (and its caller's per-atom sum, +0)
             if not self._stress:
@@ -163,5 +180,4 @@ class BispectrumBase:
                 res["rdxdr"] = np.zeros((k, tab.nB, 6))
             else:
                 res["rdxdr"] = -np.zeros((pk, tab.nB, 3, 3)) / vol
-        self.clear_memory()
-        return res
+        return res, nb

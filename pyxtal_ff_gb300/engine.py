@@ -34,6 +34,58 @@ def require_cuda():
         raise RuntimeError("pyxtal_ff_gb300 needs a CUDA GPU (GB300, sm_103a); there is no CPU fallback")
 
 
+# Host copies go through pinned memory (torch's cached pinned blocks, about STAGE_BYTES of them in use
+# per call at most) and large ones are spread over the CPU's threads: a copy straight into new pageable
+# memory is bound by its page faults, which one thread takes (results that are kept: 5 MB 464 us,
+# staged 70; 20 MB 2,909 and 226 us), and each such copy is a wait of its own (12.6 us).
+STAGE_BYTES = 16 << 20
+_ONE_THREAD_BYTES = 256 << 10
+
+
+def _unpin(h):
+    if h.numel() * h.element_size() <= _ONE_THREAD_BYTES:
+        return h.numpy().copy()
+    return torch.empty(h.shape, dtype=h.dtype).copy_(h).numpy()
+
+
+def to_host(*tensors):
+    """New numpy arrays with the values of device tensors (None stays None), read with one wait
+    where they fit the staging memory together, else each through its two halves in turn."""
+    src = [None if t is None else t.detach().contiguous() for t in tensors]
+    dev = [s for s in src if s is not None and s.device.type != "cpu"]
+    out = [s if s is None or s.device.type != "cpu" else s.numpy() for s in src]
+    if not dev:
+        return out
+    stream = torch.cuda.current_stream(dev[0].device)
+    if sum(s.numel() * s.element_size() for s in dev) <= STAGE_BYTES:
+        pinned = [torch.empty(s.shape, dtype=s.dtype, pin_memory=True).copy_(s, non_blocking=True) for s in dev]
+        stream.synchronize()
+        done = [_unpin(h) for h in pinned]
+    else:
+        done = _read_large(dev, stream)
+    got = iter(done)
+    return [next(got) if isinstance(o, torch.Tensor) else o for o in out]
+
+
+def _read_large(dev, stream):
+    out = [torch.empty(s.shape, dtype=s.dtype) for s in dev]
+    half = STAGE_BYTES // 2
+    stage = torch.empty((2, half), dtype=torch.uint8, pin_memory=True)
+    events = [torch.cuda.Event(), torch.cuda.Event()]
+    flat = [(s.view(-1).view(torch.uint8), o.view(-1).view(torch.uint8)) for s, o in zip(dev, out) if s.numel()]
+    pieces = [(s[a:a + half], o[a:a + half]) for s, o in flat for a in range(0, s.numel(), half)]
+    for k in range(len(pieces) + 1):
+        if k < len(pieces):
+            s = pieces[k][0]
+            stage[k & 1, : s.numel()].copy_(s, non_blocking=True)
+            events[k & 1].record(stream)
+        if k > 0:  # the piece before, while this one is on its way
+            events[(k - 1) & 1].synchronize()
+            o = pieces[k - 1][1]
+            o.copy_(stage[(k - 1) & 1, : o.numel()])
+    return [o.numpy() for o in out]
+
+
 # ---------------------------------------------------------------------- tables
 class Tables:
     """Device-resident CG / rootpq / index tables for one (twol, normalize_U), built for
@@ -317,6 +369,34 @@ def build_neighbors(pos, cells, pbc, atom_ptr, rcut, device="cuda", workspace=No
     return neighbors_view(lay, bufs, M, P, bits)
 
 
+def start_neighbors(pos, cells, pbc, atom_ptr, rcut, device="cuda"):
+    """build_neighbors without its wait: (record with the capacities as counts, finish).  Kernels that
+    take a capacity for the number of images may be launched on the record at once (a list that
+    overflows its buffers is left empty); finish() then waits for the list alone and returns the
+    record with the true counts, or None where the list did not fit and has to be built again."""
+    dev = torch.device(device)
+    lay = layout(cells, pbc, atom_ptr, rcut, dev)
+    if pos.shape != (lay.natoms, 3):
+        raise ValueError("positions must be (N,3) for N = atom_ptr[-1]")
+    cap_m, cap_p = capacity_for(lay)
+    bufs = NeighborBuffers.allocate(lay, cap_m, cap_p, dev)
+    enqueue_neighbors(lay, pos, bufs)
+    host = torch.empty(3, dtype=torch.int32, pin_memory=True)
+    host.copy_(bufs.summary_dev(), non_blocking=True)
+    done = torch.cuda.Event()
+    done.record(torch.cuda.current_stream(dev))
+
+    def finish():
+        done.synchronize()
+        M, P, bits = host.tolist()
+        if not check_summary(M, P, bits, cap_m, cap_p):
+            return None
+        note_capacity(lay, M, P)
+        return neighbors_view(lay, bufs, M, P, bits)
+
+    return neighbors_view(lay, bufs, cap_m, cap_p), finish
+
+
 # ----------------------------------------------------------------- compute
 def site_weights(kind, numbers, symbols, weights=None):
     """(w_nb, w_site) per atom: SO4.py uses atomic numbers for both
@@ -392,10 +472,15 @@ def contract_dxdr(beta, pair_ptr, seq, atom_struct, atom_ptr, dxdr=None, rdxdr_a
     check(lib().so4_contract_dxdr(prec, natoms, nB, nstruct, _ptr(keep[3]), _ptr(keep[4]), _ptr(keep[1]),
                                   _ptr(keep[2]), _ptr(keep[5]), _ptr(keep[0]), _ptr(keep[6]), _ptr(forces), _ptr(sa),
                                   _ptr(stress), _ptr(status), _stream()), "so4_contract_dxdr")
-    bits = int(status.item()) if own else 0
+    if own:
+        check_contract(int(status.item()))
+    return (forces[:natoms] if forces is not None else None), (stress[:nstruct] if stress is not None else None)
+
+
+def check_contract(bits):
+    """Raise for the status bits of contract_dxdr."""
     if bits & (1 << _lib.SO4_ERR_REVERSE):
         raise ValueError("so4_contract_dxdr: a pair has no reverse pair (the pair list is not symmetric)")
-    return (forces[:natoms] if forces is not None else None), (stress[:nstruct] if stress is not None else None)
 
 
 def design_forces(X, ncols, nB, nelem, species, pair_ptr, seq, atom_struct, atom_ptr, dxdr, force_row):

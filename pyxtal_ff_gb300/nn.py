@@ -89,6 +89,12 @@ class NeuralNetworkPotential:
         descriptor: the plain path's dict -- x (N, nB), dxdr (P, nB, 3), seq (P, 2),
         rdxdr (N, nB, 6) per-atom Voigt rows (the caller's reduction), elements --
         as numpy arrays or device tensors."""
+        d = self._device_properties(descriptor, bforce, bstress)
+        return self._host_properties(*engine.to_host(*d), n=d[0].shape[0])
+
+    def _device_properties(self, descriptor, bforce, bstress, pair_ptr=None):
+        """energies, forces, stress (not yet in GPa) and the contraction's status word on the device
+        (None where not asked for); pair_ptr (N + 1,) i32: the pairs of each centre, where known."""
         dev = self.device
 
         def dev64(a):
@@ -97,24 +103,28 @@ class NeuralNetworkPotential:
         x = dev64(descriptor["x"])
         n = x.shape[0]
         energies, _, dedx = self.energies_and_dedx(x, descriptor["elements"])
-        forces = np.zeros((n, 3))
-        stress = np.zeros(6)
-        if (bforce or bstress) and n > 0:
-            seq = torch.as_tensor(descriptor["seq"]).to(dev, dtype=torch.int64).contiguous()
+        if not (bforce or bstress) or n == 0:
+            return energies, None, None, None
+        seq = torch.as_tensor(descriptor["seq"]).to(dev, dtype=torch.int64).contiguous()
+        if pair_ptr is None:
             counts = torch.bincount(seq[:, 0], minlength=n)
             pair_ptr = torch.cat([torch.zeros(1, dtype=torch.int64, device=dev), torch.cumsum(counts, 0)]).int()
-            atom_struct = torch.zeros(n, dtype=torch.int32, device=dev)
-            atom_ptr = torch.tensor([0, n], dtype=torch.int32, device=dev)
-            fscale = BOHR if self.unit == "Ha" else 1.0
-            sscale = BOHR ** 3 if self.unit == "Ha" else 1.0
-            dxdr = dev64(descriptor["dxdr"]) * fscale if bforce else None
-            rd = dev64(descriptor["rdxdr"]) * sscale if bstress else None
-            f, s = engine.contract_dxdr(dedx, pair_ptr, seq, atom_struct, atom_ptr, dxdr=dxdr, rdxdr_atom=rd)
-            if f is not None:
-                forces = f.cpu().numpy()
-            if s is not None:
-                stress = s[0].cpu().numpy() * EV2GPA
-        return energies.cpu().numpy(), forces, stress
+        atom_struct = torch.zeros(n, dtype=torch.int32, device=dev)
+        atom_ptr = torch.tensor([0, n], dtype=torch.int32, device=dev)
+        status = torch.zeros(1, dtype=torch.int32, device=dev)
+        dxdr = dev64(descriptor["dxdr"]) if bforce else None
+        rd = dev64(descriptor["rdxdr"]) if bstress else None
+        if self.unit == "Ha":
+            dxdr = dxdr * BOHR if bforce else None
+            rd = rd * BOHR ** 3 if bstress else None
+        f, s = engine.contract_dxdr(dedx, pair_ptr, seq, atom_struct, atom_ptr, dxdr=dxdr, rdxdr_atom=rd, status=status)
+        return energies, f, s, status
+
+    @staticmethod
+    def _host_properties(energies, f, s, status, n):
+        if status is not None:
+            engine.check_contract(int(status[0]))
+        return energies, (np.zeros((n, 3)) if f is None else f), (np.zeros(6) if s is None else s[0] * EV2GPA)
 
     @property
     def no_of_descriptors(self):

@@ -69,7 +69,7 @@ class Atoms:
 
     @property
     def symbols(self):
-        return [CHEMICAL_SYMBOLS[z] for z in self.numbers]
+        return [CHEMICAL_SYMBOLS[z] for z in self.numbers.tolist()]
 
     def get_chemical_symbols(self):
         return self.symbols
@@ -99,7 +99,7 @@ def as_arrays(atoms):
         pbc = atoms.get_pbc()
     pbc = np.array(np.broadcast_to(np.asarray(pbc, dtype=bool), (3,)), dtype=np.int32)
     numbers = np.asarray(atoms.numbers, dtype=np.int64)
-    symbols = [str(s) for s in list(atoms.symbols)]
+    symbols = list(map(str, atoms.symbols))
     return pos, cell, pbc, numbers, symbols
 
 
