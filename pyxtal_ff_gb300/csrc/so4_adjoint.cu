@@ -234,7 +234,7 @@ struct ZLArgs {
     const int *jbase, *jpos;
     const float *jfac;
     const float *yscale;  // n_half: Y is stored times the row scale F of its entry
-    int parts;            // k_zw64: CTAs (a cluster) per group of atoms
+    int full, parts;      // k_zw64: groups of one CTA, CTAs (a cluster) of each other group
     int stage_cap;        // MODE 3: slot rows the epilogue stages at a time (those fitting over the U tiles)
 };
 
@@ -638,14 +638,17 @@ __device__ __forceinline__ void zw2_unit_k(int k, const ZLArgs &A, const int4 un
 
 // k_zw32 with two atoms per lane: 64 atoms per CTA of NT threads, one CTA per SM (the
 // two-atom U tiles of twol 8 take 155 KB).  The same work lists, modes and outputs.
-// A cluster of A.parts CTAs shares a group of 64 atoms, CTA r taking units r, r + parts, ..;
-// the slot sums follow a cluster barrier, in CTA 0 (zw_parts below).
-template <int MODE, bool CA_SMEM, int NT>
-__global__ void __launch_bounds__(NT, 1) k_zw64(ZLArgs A) {
+// The first A.full groups of 64 atoms have a CTA each; the others are shared by clusters of
+// A.parts CTAs, CTA r taking units r, r + parts, .., and the slot sums follow a cluster barrier,
+// in CTA 0 (zw_split below).
+template <int MODE, bool CA_SMEM, int NT, int NCTA = 1>
+__global__ void __launch_bounds__(NT, NCTA) k_zw64(ZLArgs A) {
     extern __shared__ __align__(16) float4 zw2_smem[];
     __shared__ int s_unit;
     const int lane = threadIdx.x & 31;
-    const int rank = blockIdx.x % A.parts, a0 = (int)(blockIdx.x / A.parts) * ZW2_ATOMS, a = a0 + lane;
+    const int split = (int)blockIdx.x - A.full, parts = split < 0 ? 1 : A.parts;
+    const int rank = split < 0 ? 0 : split % parts;
+    const int a0 = (split < 0 ? (int)blockIdx.x : A.full + split / parts) * ZW2_ATOMS, a = a0 + lane;
     float4 *Uq = zw2_smem;
     const size_t ntile = (size_t)(A.nu + 2 * ZW_PAD) * ZL_PITCH;  // float4
     float2 *coef = reinterpret_cast<float2 *>(zw2_smem + ntile);  // [nblk][33] pairs, MODE 1 and 2
@@ -721,13 +724,13 @@ __global__ void __launch_bounds__(NT, 1) k_zw64(ZLArgs A) {
     const float *ca = CA_SMEM ? ca_s : A.wca;
     __syncthreads();
     const float4 *Ul = Uq + lane;
-    for (int v = zl_next(&s_unit), u; (u = rank + A.parts * v) < A.nunit; v = zl_next(&s_unit)) {
+    for (int v = zl_next(&s_unit), u; (u = rank + parts * v) < A.nunit; v = zl_next(&s_unit)) {
         const int4 un = __ldg(A.unit + u);
         zw2_unit_k<MODE>(un.x >> 24, A, un, Ul, coef, ca, a, lane);
     }
     pdl_trigger();
     if (MODE == 1) return;
-    if (A.parts > 1) {
+    if (parts > 1) {
         cluster_sync();  // the other CTAs' slots are in L2, where the sums read them
         if (rank > 0) return;
     } else {
@@ -1341,37 +1344,58 @@ void so4_zw_smem_modes(const so4_tables *t, size_t out[4]) {
     out[3] = zw_smem_bytes(t, 0, false);  // the JVP stages its slots in chunks over the U tiles
 }
 
-// CTAs per group of 64 atoms, while there are fewer groups than SMs: as many as leave each
-// scheduler of an SM a unit, eight (a portable cluster) at most.  All of them run at once: a
-// cluster lies in one of the eight GPCs, each of which may leave parts - 1 SMs over.  Past that
-// the split loses (1,000 atoms of lmax 4 in 8 parts 97 us, in 6 parts 59: the last clusters wait
-// for the first).  B + Y alone at lmax 4, one CTA per group and now: 64 atoms 121 and 53 us,
-// 1,000 atoms 123 and 59, 2,744 atoms 123 and 76, 4,096 atoms 123 and 85; at lmax 3: 64 atoms
-// 39 and 28 us, 2,744 atoms 40 and 32.
+// The groups that one CTA each would leave in a last, partly filled wave (all of them, if there are
+// fewer groups than SMs) are shared by clusters: as many CTAs as leave each scheduler of an SM a
+// unit, eight (a portable cluster) at most.  All of them run at once: a cluster lies in one of the
+// eight GPCs, each of which may leave parts - 1 SMs over.  Past that the split loses (1,000 atoms
+// of lmax 4 in 8 parts 97 us, in 6 parts 59: the last clusters wait for the first).  Behind full
+// waves, whose CTAs come in clusters then too, only pairs fill all SMs.  B + Y at lmax 4, one CTA
+// per group and now: 64 atoms 121 and 53 us, 1,000 atoms 123 and 59, 2,744 atoms 123 and 76, 4,096
+// atoms 123 and 85, 12,800 atoms 250 and 214, 24,000 atoms 372 and 335; at lmax 3: 64 atoms 39 and
+// 28 us, 2,744 atoms 40 and 32.
 constexpr int ZW_SMS = 152, ZW_GPCS = 8;
-static int zw_parts(int nunit, int groups) {
-    int parts = 1;
-    for (int p = 2; p <= std::min(8, (nunit + 3) / 4); ++p)
-        if (p * groups <= ZW_SMS - ZW_GPCS * (p - 1)) parts = p;
-    return parts;
+static void zw_split(ZLArgs &Z, int groups) {
+    Z.full = groups / ZW_SMS * ZW_SMS;
+    Z.parts = 1;
+    const int rest = groups - Z.full;
+    for (int p = 2; p <= std::min(Z.full ? 2 : 8, (Z.nunit + 3) / 4); ++p)
+        if (p * rest <= ZW_SMS - ZW_GPCS * (p - 1)) Z.parts = p;
+    if (rest == 0) Z.parts = 1;
 }
 
 // k_zw64 with NT threads, the Ca table in shared memory when the one CTA per SM still
 // fits with it
+//
+// With 512 threads a CTA owns its SM, which waits while the CTA loads its tiles, at its last unit
+// and in its sums.  Where two CTAs' tiles fit (twol <= 6) and there are more groups than SMs, two
+// CTAs of 256 threads share the SM instead and fill these waits for each other.  512 and 2 x 256
+// threads, B + Y / Y / JVP: 608 groups at lmax 2 69 / 45 / 55 us and 48 / 32 / 37, at lmax 3
+// 171 / 133 / 167 and 144 / 123 / 149; 160 groups at lmax 3 81 / 61 / 80 and 71 / 60 / 73.  With
+// one group per SM it loses (lmax 3 43 and 50 us), and in the third wave, where half of the pairs'
+// places stay empty, Y alone does from lmax 2.5 on (360 groups at lmax 3 124 / 96 / 122 and
+// 118 / 97 / 119).
 template <int MODE, int NT>
 static int launch_zw64(const so4_tables *t, ZLArgs Z, int natoms, size_t smz, cudaStream_t st) {
     const size_t with_ca = smz + 16 + sizeof(float) * (size_t)t->n_wca;
     const int groups = (natoms + ZW2_ATOMS - 1) / ZW2_ATOMS;
-    Z.parts = zw_parts(Z.nunit, groups);
     int rc;
+    const bool third = MODE == 1 && t->twol > 4 && groups > 2 * ZW_SMS && groups <= 3 * ZW_SMS;
+    if (NT == 512 && groups > ZW_SMS && !third && 2 * (with_ca + 1024 + 16) <= 228 * 1024) {
+        Z.full = groups;
+        rc = set_smem(k_zw64<MODE, true, 256, 2>, with_ca);
+        if (rc) return rc;
+        return so4_launch_pdl(k_zw64<MODE, true, 256, 2>, dim3(groups), dim3(256), with_ca, st, Z);
+    }
+    zw_split(Z, groups);
+    const dim3 grid(Z.full + (groups - Z.full) * Z.parts);
     if (with_ca <= 227 * 1024) {
         rc = set_smem(k_zw64<MODE, true, NT>, with_ca);
         if (rc) return rc;
-        return so4_launch_cluster(k_zw64<MODE, true, NT>, dim3(groups * Z.parts), dim3(NT), with_ca, Z.parts, st, Z);
+        return so4_launch_cluster(k_zw64<MODE, true, NT>, grid, dim3(NT), with_ca, Z.parts, st, Z);
     }
     rc = set_smem(k_zw64<MODE, false, NT>, smz);
     if (rc) return rc;
-    return so4_launch_cluster(k_zw64<MODE, false, NT>, dim3(groups * Z.parts), dim3(NT), smz, Z.parts, st, Z);
+    return so4_launch_cluster(k_zw64<MODE, false, NT>, grid, dim3(NT), smz, Z.parts, st, Z);
 }
 
 // Launch the window kernel of the tables' layout: k_zw64 (two atoms per lane) or k_zw32

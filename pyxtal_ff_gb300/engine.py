@@ -39,7 +39,7 @@ def require_cuda():
 # memory is bound by its page faults, which one thread takes (results that are kept: 5 MB 464 us,
 # staged 70; 20 MB 2,909 and 226 us), and each such copy is a wait of its own (12.6 us).
 STAGE_BYTES = 16 << 20
-_ONE_THREAD_BYTES = 256 << 10
+_ONE_THREAD_BYTES = 512 << 10  # numpy against the parallel copy: 64 KB 2.8 and 7.4 us, 512 KB 12.9 and 14.6, 1 MB 25 and 14
 
 
 def _unpin(h):
