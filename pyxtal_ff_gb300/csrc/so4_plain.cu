@@ -78,7 +78,7 @@ struct PlainArgs {
     T *x, *dxdr, *rdxdr;
     // scratch of this pass, centre c = a - a0 in tile c / 32, lane c % 32:
     pc<T> *ut;       // U_tot, full rows: [tile][n_u][32]
-    pc<T> *zt;       // Z': [tile][n_z][32]
+    pc<T> *zt;       // Z': [tile][32 / ZQ][n_z][ZQ]
     float2 *uh;      // FP32: U_tot, half layout [centre][n_half]
     longlong2 *zi;   // k_plain_d64 without room for them in shared memory: integers [centre][n_z]
 };
@@ -283,6 +283,18 @@ __device__ __forceinline__ void plain_rows32(const SmallTables &st, const float 
 }
 
 // ---------------------------------------------------------------- Z' and B
+// Z' of centre c of the pass: its elements stand ZQ apart, those of ZQ centres side by side, a
+// sector of 32 bytes.  k_plain_z stores a centre per lane, the derivative kernels gather one
+// centre's elements.  8,000 atoms, k_plain_z + k_plain_d at ZQ = 32 / a sector / 1: FP32 lmax 3
+// 405 / 391 / 414 us, lmax 4 1,248 / 1,081 / 1,178; FP64 lmax 3 2,193 / 2,214 / 2,216, lmax 4
+// 5,590 / 5,490 / 5,477.
+template <typename T>
+constexpr int ZQ = 32 / sizeof(pc<T>);
+template <typename T>
+__device__ __forceinline__ pc<T> *plain_zt(const PlainArgs<T> &A, int c) {
+    return A.zt + (size_t)(c / ZQ<T>) * ZQ<T> * A.n_z + c % ZQ<T>;
+}
+
 // One Z unit (so4_tables.cu) of 32 centres, lane = centre, for N levels: the products
 // V_l1 V_l2 are formed once for all of them.
 template <typename T, int N>
@@ -320,7 +332,7 @@ __device__ __forceinline__ void plain_z_unit(const int4 q0, const int4 q1, const
     }
     const int out[PZ_G] = {q1.z, q1.w, q2.x, q2.y};
 #pragma unroll
-    for (int j = 0; j < N; ++j) Z[(size_t)out[j] * 32] = {zr[j], zi[j]};
+    for (int j = 0; j < N; ++j) Z[(size_t)out[j] * ZQ<T>] = {zr[j], zi[j]};
 }
 
 constexpr int ZT = 256;  // threads of k_plain_z
@@ -330,7 +342,7 @@ template <typename T>
 __global__ void __launch_bounds__(ZT) k_plain_z(PlainArgs<T> A) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const pc<T> *U = A.ut + (size_t)blockIdx.x * A.n_u * 32 + lane;
-    pc<T> *Z = A.zt + (size_t)blockIdx.x * A.n_z * 32 + lane;
+    pc<T> *Z = plain_zt(A, blockIdx.x * 32 + lane);
     for (int u = wid + (ZT / 32) * blockIdx.y; u < A.n_unit; u += (ZT / 32) * gridDim.y) {
         const int4 q0 = __ldg(A.unit + 3 * u), q1 = __ldg(A.unit + 3 * u + 1), q2 = __ldg(A.unit + 3 * u + 2);
         switch (q0.y >> 16) {
@@ -352,19 +364,27 @@ __global__ void __launch_bounds__(256) k_plain_b(PlainArgs<T> A) {
     const int4 b = __ldg(A.blk + __ldg(A.bblk + k));
     const int lam = b.w, cnt = b.z;
     const pc<T> *u = A.ut + ((size_t)blockIdx.x * A.n_u + A.st.u_block[lam]) * 32 + lane;
-    const pc<T> *z = A.zt + ((size_t)blockIdx.x * A.n_z + b.y) * 32 + lane;
+    const pc<T> *z = plain_zt(A, blockIdx.x * 32 + lane) + (size_t)b.y * ZQ<T>;
     T s = T(0);
     const int full = (lam & 1) ? cnt : cnt - 1;
 #pragma unroll 4
     for (int e = 0; e < full; ++e) {
-        const pc<T> p = u[(size_t)e * 32], q = z[(size_t)e * 32];
+        const pc<T> p = u[(size_t)e * 32], q = z[(size_t)e * ZQ<T>];
         s = fma(p.re, q.re, fma(p.im, q.im, s));
     }
     if (full < cnt) {
-        const pc<T> p = u[(size_t)full * 32], q = z[(size_t)full * 32];
+        const pc<T> p = u[(size_t)full * 32], q = z[(size_t)full * ZQ<T>];
         s += T(0.5) * (p.re * q.re + p.im * q.im);
     }
     if (a < A.natoms) A.x[(size_t)a * A.n_b + k] = T(2) * s;
+}
+
+// 1 / v in FP32, from v = vh + vl: the quotient of vh corrected by its residual, within a few
+// thousandths of half an ulp.  (An FP64 division is some thirty instructions of a pipe with 1/64
+// of the FP32 rate, in the one warp that the CTA waits for.)
+__device__ __forceinline__ float inv32(double v) {
+    const float vh = (float)v, vl = (float)(v - (double)vh), y = 1.f / vh;
+    return fmaf(fmaf(-vl, y, fmaf(-vh, y, 1.f)), y, y);
 }
 
 // ---------------------------------------------------------------- dB/dr
@@ -575,7 +595,7 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
     const int CB = L.cb;
     pc<double> *V = (pc<double> *)smem_raw;
     longlong2 *Vi = (longlong2 *)V;
-    const pc<double> *Zt = A.zt + (size_t)(c >> 5) * nz * 32 + (c & 31);
+    const pc<double> *Zt = plain_zt(A, c);
     longlong2 *Zi = ZS ? (longlong2 *)(smem_raw + L.z) : A.zi + (size_t)c * nz;
     unsigned *Cl = (unsigned *)(smem_raw + L.c);
     int *Ch = (int *)Cl + 4 * VI * CB;
@@ -621,7 +641,7 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
             for (int r = 0; r < RQ; ++r) {
                 const int q = q0 + r * NQ + tid - 32;
                 ze[r] = q < nz ? __ldg(A.zent + q) : -1;
-                if (q < nz) v[r] = Zt[(size_t)q * 32];
+                if (q < nz) v[r] = Zt[(size_t)q * ZQ<double>];
             }
 #pragma unroll
             for (int r = 0; r < RQ; ++r) {
@@ -924,6 +944,7 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
     __shared__ SmallTables st;
     __shared__ PlainRuns R;
     __shared__ int s_comp;
+    __shared__ float inv_s;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     if (tid == 0) st = A.st;
     const int nB = A.n_b, c = blockIdx.x, a = A.a0 + c;
@@ -933,7 +954,7 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
     float4 *W = (float4 *)(smem_raw + L.w);
     int *vrow = (int *)(smem_raw + L.vrow);
     float *t3 = (float *)(smem_raw + L.t), *par = (float *)(smem_raw + L.par);
-    const pc<float> *Zt = A.zt + (size_t)(c >> 5) * A.n_z * 32 + (c & 31);
+    const pc<float> *Zt = plain_zt(A, c);
     const int m0 = A.img_ptr[a], m1 = A.img_ptr[a + 1], p0 = A.pair_ptr[a], ns = A.nsite[a];
     const bool self_img = A.pair_img[ns] < A.pair_img[ns + 1];
     // the (i, i) row takes the centre's own images as they come
@@ -950,8 +971,8 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
         for (int e = w0 + t0; e < w1; e += nt) {
             const int4 ps = __ldg(A.wpos + e);
             const float4 f = __ldg(A.wfac + e);
-            const pc<float> z = Zt[(size_t)ps.x * 32], zq = Zt[(size_t)ps.z * 32];
-            pc<float> zn = Zt[(size_t)ps.y * 32];
+            const pc<float> z = Zt[(size_t)ps.x * ZQ<float>], zq = Zt[(size_t)ps.z * ZQ<float>];
+            pc<float> zn = Zt[(size_t)ps.y * ZQ<float>];
             if (ps.w & 1) zn.re = -zn.re;  // the mirror -conj(Z'[m-1]) past a middle row's centre
             const float xr = f.z * zn.re, xi = f.z * zn.im, yr = f.w * zq.re, yi = f.w * zq.im;
             // (re of W0..W3), (im of W0..W3)
@@ -960,12 +981,13 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
             vrow[e - w0] = (ps.w >> 1) * P;
         }
     };
+    float s_inv = 0.f;  // 1 / volume: warp 0's, the others read inv_s
     auto setup = [&](int base, int n) {  // warp 0
         const int m = base + lane;
         const int j = lane < n ? A.img_j[m] : -1;
         const bool fresh = lane < n && (m == m0 || A.img_j[m - 1] != j);
         float ck[4], q[12], rv[3];
-        plain_image<float>(A, a, m, lane < n, (float)(1.0 / A.geom[A.astruct[a]].vol), j, ck, q, rv);
+        plain_image<float>(A, a, m, lane < n, s_inv, j, ck, q, rv);
 #pragma unroll
         for (int i = 0; i < 4; ++i) par[32 * i + lane] = ck[i];
 #pragma unroll
@@ -975,7 +997,11 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
         plain_runs(R, n, 32, j, fresh, a, p0, self_img, npair);
     };
     // the first images' set-up (warp 0) beside the first batch's W (the others)
-    if (wid == 0) setup(m0, min(32, m1 - m0));
+    if (wid == 0) {
+        s_inv = inv32(A.geom[A.astruct[a]].vol);
+        if (lane == 0) inv_s = s_inv;
+        setup(m0, min(32, m1 - m0));
+    }
     else form(0, tid - 32, ST - 32);
     int have = 0;  // the batch the buffer holds
     const int sub = lane >> 3, il = lane & 7;
@@ -1101,7 +1127,7 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
         __syncthreads();
     }
     // ---- the (i, i) row: minus the sum of the others
-    const float inv_vol = (float)(1.0 / A.geom[A.astruct[a]].vol);
+    const float inv_vol = inv_s;
     float *Ds = (float *)smem_raw;
 #pragma unroll
     for (int s = 0; s < KS; ++s) {
@@ -1133,8 +1159,6 @@ bool d64_zs(const so4_tables *t) {
     return with <= TWO_CTAS || (without > TWO_CTAS && with <= ONE_CTA);
 }
 
-// A tile's Z units are spread over up to n_unit / 16 CTAs while the grid has fewer than eight
-// CTAs per SM: 64 centres (two tiles) at lmax 3 would otherwise run on two SMs.
 // Scratch per 32 centres, and the centres of one pass: all of them, or what fits in PLAIN_BYTES.
 constexpr size_t PLAIN_BYTES = (size_t)768 << 20;
 
@@ -1235,6 +1259,8 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
             k_plain_tile<<<nt, 256, 0, st>>>(A);
         }
         // a tile's units over as many CTAs as it takes to give every SM several
+        // A tile's Z units are spread over up to n_unit / 16 CTAs while the grid has fewer than eight
+        // CTAs per SM: 64 centres (two tiles) at lmax 3 would otherwise run on two SMs.
         const int parts = std::max(1, std::min((A.n_unit + 15) / 16, 1216 / nt));
         k_plain_z<T><<<dim3(nt, parts), ZT, 0, st>>>(A);
         k_plain_b<T><<<dim3(nt, (t->n_b + 7) / 8), 256, 0, st>>>(A);
