@@ -42,6 +42,13 @@ class LinearModel(torch.nn.Module):
         return (x * self.coef[species]).sum(-1) + self.bias[species]
 
 
+# Up to 152 groups of 64 atoms the window kernel of one branch spreads over the whole chip, and a second
+# branch only gets in its way; with more, one branch's kernels fill what the other's last waves leave.
+# One and two branches: lmax 3 2,744 atoms 126 and 139 us, 8,000 188 and 191, 10,648 251 and 226; lmax 4
+# 1,000 atoms 139 and 176 us, 8,000 299 and 312, 10,648 412 and 415, 13,824 472 and 450.
+TWO_BRANCH_ATOMS = 64 * 152
+
+
 class Batch:
     """Host description of a batch of structures (cells, pbc, atom ranges, species)."""
 
@@ -139,9 +146,12 @@ class SO4Calculator:
     def capture(self, batch: Batch, model, headroom=1.25, branches=None, pdl=None, host_io=False):
         """The whole energy / forces / stress step of this batch layout as one CUDA graph
         (see CapturedStep); call the result with new positions.  branches / pdl default to
-        the calculator's tuning (2 and off untuned); host_io: the graph also copies the
-        positions in from, and the results out to, pinned host buffers of the step."""
-        return CapturedStep(self, batch, model, headroom=headroom, branches=self.branches if branches is None else branches,
+        the calculator's tuning (untuned: 2 above TWO_BRANCH_ATOMS, else 1, and off); host_io: the
+        graph also copies the positions in from, and the results out to, pinned host buffers of
+        the step."""
+        if branches is None:
+            branches = self.branches if self.tuning is not None or batch.natoms > TWO_BRANCH_ATOMS else 1
+        return CapturedStep(self, batch, model, headroom=headroom, branches=branches,
                             pdl=self.pdl if pdl is None else pdl, host_io=host_io)
 
     def neighbors(self, batch: Batch, positions):
@@ -312,6 +322,7 @@ class CapturedStep:
             self.bc = [torch.empty((max(tab.n_bsec, 1), a1 - a0), dtype=torch.float32, device=dev)
                        for a0, a1 in self.chunks]
         self.sides = [torch.cuda.Stream(device=dev) for _ in range(self.branches - 1)]
+        self.reverse = torch.cuda.Stream(device=dev)
         self.host_io = bool(host_io)
         if self.host_io:
             self.host_positions = torch.from_numpy(np.ascontiguousarray(batch.positions, dtype=np.float64)).pin_memory()
@@ -352,11 +363,10 @@ class CapturedStep:
         return buf[:S], buf[S:S + 3 * N].view(N, 3), buf[S + 3 * N:].view(S, 6)
 
     def _enqueue_linear(self):
-        lay, calc, tab, L = self.layout, self.calc, self.calc.tables, engine.lib()
+        calc, tab, L = self.calc, self.calc.tables, engine.lib()
         b = self.nl
         _p = engine._ptr
         check = engine.check
-        N, S_ = lay.natoms, lay.nstruct
 
         def compute(a0, a1, bc):
             """U_tot, B and Y, and the per-image dE/dr of one range of centres."""
@@ -370,46 +380,56 @@ class CapturedStep:
                                          _p(b.img_ptr[a0:a1 + 1]), _p(b.img_j), _p(b.img_r), self.cap_m,
                                          _p(self.ybuf[a0:a1]), _p(self.g), s_), "so4_adjoint_deidrj32")
 
-        if self.branches == 1:
+        self._lists(lambda k, a0, a1: compute(a0, a1, self.bc[k]))
+        self._gather(self.bias_s)
+
+    def _lists(self, compute):
+        """The neighbour list, and compute(k, a0, a1) on the centres of branch k behind their part of it.
+
+        Bins for all atoms first; then each branch counts and sorts its own centres (their scans
+        chained in branch order) and goes on to its compute while the other branches' lists are
+        still being built.  The reverse images, read only by the gather, are found beside the
+        compute of a single branch on a stream of their own (64 atoms 96.3 -> 92.7 us; 32,000 atoms
+        in two branches 908 -> 914: there they follow the join); the summary comes last."""
+        lay, L, b, _p, check = self.layout, engine.lib(), self.nl, engine._ptr, engine.check
+        N, S_, G = lay.natoms, lay.nstruct, lay.nbins
+        if not self.chunks:
             engine.enqueue_neighbors(lay, self.pos, b, lite=True, count_pairs=False)
-            for (a0, a1), bc in zip(self.chunks, self.bc):
-                compute(a0, a1, bc)
-        else:
-            # the list itself runs per branch: bins for all atoms, then each branch counts and
-            # sorts its own centres (their scans chained in branch order) and goes on to its
-            # compute while the other branches' lists are still being built; the reverse images
-            # (read only by the gather) and the summary follow the join
-            G = lay.nbins
-            check(L.so4_nl_bins(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N, b.slot_cap, _p(b.ws),
-                                b.ws.numel(), engine._stream()), "so4_nl_bins")
-            main = torch.cuda.current_stream()
-            for sd in self.sides:
-                sd.wait_stream(main)
-            scanned = None
-            for (a0, a1), bc, st in zip(self.chunks, self.bc, [main] + self.sides):
-                with torch.cuda.stream(st):
-                    s_ = engine._stream()
-                    check(L.so4_nl_count_keys_range(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N,
-                                                    lay.rcut, b.slot_cap, a0, a1, _p(b.ws), b.ws.numel(), s_),
-                          "so4_nl_count_keys_range")
-                    if scanned is not None:
-                        st.wait_event(scanned)
-                    check(L.so4_nl_scan_range(N, G, b.slot_cap, a0, a1, _p(b.img_ptr), _p(b.ws), b.ws.numel(), s_),
-                          "so4_nl_scan_range")
-                    scanned = torch.cuda.Event()
-                    scanned.record(st)
-                    check(L.so4_nl_sort_range(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N, a0, a1,
-                                              _p(b.img_ptr), b.cap_m, b.slot_cap, _p(b.img_j), _p(b.img_off),
-                                              _p(b.img_r), _p(b.ws), b.ws.numel(), s_), "so4_nl_sort_range")
-                    compute(a0, a1, bc)
-            for sd in self.sides:
-                main.wait_stream(sd)
+            return
+        check(L.so4_nl_bins(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N, b.slot_cap, _p(b.ws),
+                            b.ws.numel(), engine._stream()), "so4_nl_bins")
+        main = torch.cuda.current_stream()
+        for sd in self.sides:
+            sd.wait_stream(main)
+        scanned, lists = None, []
+        for k, ((a0, a1), st) in enumerate(zip(self.chunks, [main] + self.sides)):
+            with torch.cuda.stream(st):
+                s_ = engine._stream()
+                check(L.so4_nl_count_keys_range(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N,
+                                                lay.rcut, b.slot_cap, a0, a1, _p(b.ws), b.ws.numel(), s_),
+                      "so4_nl_count_keys_range")
+                if scanned is not None:
+                    st.wait_event(scanned)
+                check(L.so4_nl_scan_range(N, G, b.slot_cap, a0, a1, _p(b.img_ptr), _p(b.ws), b.ws.numel(), s_),
+                      "so4_nl_scan_range")
+                scanned = st.record_event()
+                check(L.so4_nl_sort_range(_p(lay.geom), S_, G, _p(self.pos), _p(lay.atom_struct), N, a0, a1,
+                                          _p(b.img_ptr), b.cap_m, b.slot_cap, _p(b.img_j), _p(b.img_off),
+                                          _p(b.img_r), _p(b.ws), b.ws.numel(), s_), "so4_nl_sort_range")
+                lists.append(st.record_event())
+                compute(k, a0, a1)
+        for sd in self.sides:
+            main.wait_stream(sd)
+        if self.branches == 1:
+            self.reverse.wait_event(lists[0])
+        with torch.cuda.stream(self.reverse if self.branches == 1 else main):
             check(L.so4_nl_pairs(_p(lay.geom), S_, _p(lay.atom_struct), N, _p(b.img_ptr), b.cap_m, _p(b.img_j),
                                  _p(b.img_off), _p(None), b.cap_p, _p(None), _p(None), _p(None), _p(None),
                                  _p(b.img_rev), _p(b.ws), b.ws.numel(), engine._stream()), "so4_nl_pairs")
-            check(L.so4_nl_summary(_p(b.img_ptr), _p(None), N, _p(b.ws), b.ws.numel(), engine._stream(), None),
-                  "so4_nl_summary")
-        self._gather(self.bias_s)
+        if self.branches == 1:
+            main.wait_stream(self.reverse)
+        check(L.so4_nl_summary(_p(b.img_ptr), _p(None), N, _p(b.ws), b.ws.numel(), engine._stream(), None),
+              "so4_nl_summary")
 
     def _gather(self, bias):
         """Forces, virial, energy (plus the per-structure constant) and stress, with the arithmetic of
@@ -424,10 +444,15 @@ class CapturedStep:
         """The general-model step: neighbour list, U_tot and B (so4_forward32), the model and
         beta = dE/dB by autograd, Y, the per-image dE/dr and the gather with the per-atom
         energies -- the kernels and order of SO4Calculator.compute, so the two agree bit for bit."""
-        lay, calc, tab, L = self.layout, self.calc, self.calc.tables, engine.lib()
+        self._lists(lambda k, a0, a1: self._model_beta())
+        if not self.chunks:
+            self._model_beta()
+        self._gather(None)
+
+    def _model_beta(self):
+        calc, tab, L = self.calc, self.calc.tables, engine.lib()
         b, _p, check, st = self.nl, engine._ptr, engine.check, engine._stream()
-        N, S = lay.natoms, lay.nstruct
-        engine.enqueue_neighbors(lay, self.pos, b, lite=True, count_pairs=False)
+        N = self.layout.natoms
         check(L.so4_forward32(tab.handle, C.byref(calc.params), N, _p(calc._w_nb), _p(calc._w_site), _p(b.img_ptr),
                               _p(b.img_j), _p(b.img_r), _p(self.utot), _p(self.x), _p(self.fws), self.fws.numel(), st),
               "so4_forward32")
@@ -445,7 +470,6 @@ class CapturedStep:
         check(L.so4_adjoint_deidrj32(tab.handle, C.byref(calc.params), N, _p(calc._w_nb), _p(b.img_ptr),
                                      _p(b.img_j), _p(b.img_r), self.cap_m, _p(self.ybuf), _p(self.g), st),
               "so4_adjoint_deidrj32")
-        self._gather(None)
 
     def __call__(self, positions=None):
         """One step; positions (N,3) f64 from the host (pinned for an asynchronous copy)

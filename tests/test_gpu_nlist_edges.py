@@ -10,7 +10,7 @@ import torch
 from oracle import oracle as O
 from pyxtal_ff_gb300 import engine
 from pyxtal_ff_gb300 import structures as S
-from pyxtal_ff_gb300.calculator import Batch
+from pyxtal_ff_gb300.calculator import Batch, LinearModel, SO4Calculator
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +59,25 @@ def test_neighbour_list_is_the_oracles(cuda_device, case):
         assert np.array_equal(h["pair_img"][p0:p1 + 1] - m0, ref.pair_img[: p1 - p0 + 1])
         assert np.array_equal(h["nsite"][a0:a1] - p0, ref.nsite)
         assert np.array_equal(h["img_pair"][m0:m1] - p0, np.repeat(np.arange(p1 - p0), np.diff(ref.pair_img[: p1 - p0 + 1])))
+
+
+@pytest.mark.parametrize("cells,branches", [((1, 1, 1), 1), ((19, 8, 8), 1), ((17, 13, 11), 2)])
+def test_captured_step_is_compute(cuda_device, cells, branches):
+    """The captured step (its list in one or two branches: 8, 9,728 and 19,448 atoms) against the
+    uncaptured call, bit for bit, and positions whose list outgrows the buffers (or does not:
+    the 8 atoms')."""
+    batch = Batch([_si(*cells)])
+    calc = SO4Calculator(lmax=1, rcut=4.9, kind="SNAP", weights={"Si": 1.0})
+    model = LinearModel(torch.linspace(-1, 1, calc.nB)[None]).cuda()
+    step = calc.capture(batch, model)
+    assert step.branches == branches
+    pos = batch.positions + np.random.default_rng(74).normal(0, 0.02, batch.positions.shape)
+    out, ref = step(pos), calc.compute(batch, model, positions=pos)
+    assert step.check()
+    for key in ("energy", "forces", "stress", "x"):
+        assert torch.equal(out[key], ref[key]), key
+    step(0.5 * pos)
+    nb = calc.neighbors(batch, torch.from_numpy(0.5 * pos).cuda())
+    assert step.check() == (nb.nimg <= step.cap_m and int(torch.diff(nb.img_ptr).max()) <= step.slot_cap)
+    out = step(pos)
+    assert step.check() and torch.equal(out["forces"], ref["forces"])
