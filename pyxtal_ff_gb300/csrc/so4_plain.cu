@@ -60,7 +60,7 @@ struct PlainArgs {
     int a0, natoms;  // centres a0 .. natoms - 1
     int n_u, n_half, n_z, n_b, n_blk, n_unit;
     T rc, psi_fac;  // rcut and rfac0 pi / rcut
-    int vs, cw;  // k_plain_d64: bounds 2^vs >= |V| 2^row and 2^cw >= level
+    int cw;  // k_plain_d64: 2^cw bounds the weights in W, times 4
     const so4_geom *geom;
     const int *astruct;
     const double *pos, *w_nb, *w_site, *img_r;
@@ -498,16 +498,21 @@ __device__ __forceinline__ void plain_self_row(const PlainArgs<T> &A, int a, int
 // centre, 17,768 multiply-adds per image at lmax 4 (60 % of the path's FP64 work, and FP64
 // runs at 1/64 of the FP32 rate here).  It runs on the tensor cores on integers cut into
 // signed 8-bit digits (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer.
-// Algorithms 59, 95 (2012)): V is rounded once to 61 bits relative to its bound and Z' to 59
-// relative to the component's largest entry, W formed from Z' in integers, the digits are
+// Algorithms 59, 95 (2012)): V is rounded once to 61 bits relative to its bound and Z' to 55
+// or more relative to the component's largest entry, W formed from Z' in integers, the digits are
 // exact in FP16, and the sums of the digit products p + q = s < ND stay below 2^24, exact in
 // the FP32 accumulators.  Each component's P_g is summed over its blocks as integers (any
 // order gives the same bits, so warps add with shared-memory atomics) and converted once.
+// Both integers are scaled entry by entry with the power of two next to F: with one per row the
+// rounding grew with the range of F within a row, and dB/dr at lmax 6 (lmax 4) was 5.8e-15
+// (1.9e-15) off a 64-bit evaluation instead of 2.1e-15 (1.8e-15); plain FP64 sums 1.9e-15 (1.6e-15).
 constexpr int DT = 192;    // threads: two CTAs per SM with 168 registers each
 constexpr int ND = 8;      // digits
 constexpr int VB = 61, ZB = 62;  // bits of V and W
-// The integer of P counts units of 2^66 of the product of V's and W's integers.  By the norms
-// of V's rows (and |W| <= 2^62) one block's is below 2^61, a component's three below 2^63.
+constexpr int VS = 1;  // |V| 2^exponent <= 2: |U| <= 1, and both powers of two are within sqrt(2)
+// The integer of P counts units of 2^66 of the product of V's and W's integers.  By the norms of
+// U's rows a block's |V| sum to 2^60 x 25.3 at most (twol 12), and |W| <= 2^62.5: a component's
+// three blocks stay below 2^62.8.
 constexpr int PSH = 66;
 constexpr int EMIN = -900;  // smallest exponent a component is scaled by
 constexpr int KBAD = 1 << 20;  // the exponent of a component with Inf or NaN in its Z'
@@ -658,7 +663,7 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
                     const unsigned mant = (((top >> 10) & 0x3ff) + 0x401) * (((hf >> 10) & 0x3ff) + 0x401);
                     ex = top >= 0x7ff00000u
                              ? KBAD
-                             : (int)(top >> 20) + (hf >> 20) - 2044 - (ze[r] >> 16) - (mant < (1u << 21) ? 1 : 0);
+                             : (int)(top >> 20) + (hf >> 20) - 2044 - ((ze[r] >> 16) - 64) - (mant < (1u << 21) ? 1 : 0);
                 }
                 const unsigned peers = __match_any_sync(0xffffffffu, k);
                 const int big = __reduce_max_sync(peers, ex);
@@ -668,8 +673,8 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
     }
     __syncthreads();
     const int bz = ZB - A.cw;
-    // P = integer x 2^(psh + kex), for g = 0 2^-cw less (W0 is Z' x 2^cw)
-    const int psh = PSH - (VB - A.vs) - bz;
+    // P = integer x 2^(psh + kex), for g = 0 2^-cw and else 2^-2 less (W is Z' x 2^cw, and x 4)
+    const int psh = PSH - (VB - VS) - bz;
     for (int q0 = tid; q0 < nz; q0 += 4 * DT) {
         pc<double> v[4];
         int4 bk[4];
@@ -683,7 +688,7 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
             v[r] = ((const pc<double> *)Zi)[q];
             bk[r] = __ldg(A.blk + b);
             f[r] = __ldg(A.fac + b);
-            row[r] = ze >> 16;
+            row[r] = (ze >> 16) - 64;
             ex[r] = kex[bk[r].x];
         }
 #pragma unroll
@@ -724,7 +729,7 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
             const int sh = nc > 8 ? 4 : 3;
             for (int t = tid; t < nh << sh; t += DT) {
                 const int e = t >> sh, i = t & ((1 << sh) - 1), at = v_at(e, i);
-                const int w = __ldg(&A.vent[e].w), ex = VB - A.vs + (w >> 16) - (w & 1);
+                const int w = __ldg(&A.vent[e].w), ex = VB - VS + (w >> 16) - 64 - (w & 1);
                 longlong2 z = {0, 0};
                 if (i < nc) {
                     const pc<double> v = V[at];
@@ -766,9 +771,12 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
                         const int se = __ldg(sent + ec), ma = se & 0xff;
                         const bool ctr = (se >> 8) & 1;
                         // W = p X -+ m Y: X = Y = Z'[m] (g = 0: p = 2^cw, m = 0; g = 1), else
-                        // X = Z'[m+1], Y = Z'[m-1] (at the centre X is the mirror -conj(Y)); a
-                        // neighbour past a row's end has weight 0, the clamps keep it in the block
-                        unsigned wp = g4 == 0 ? 1u << A.cw : (unsigned)(lam - ma), wm = g4 == 0 ? 0u : (unsigned)ma;
+                        // X = Z'[m+1], Y = Z'[m-1] (at the centre X is the mirror -conj(Y)), on
+                        // their own scales; a neighbour past a row's end has weight 0, the clamps
+                        // keep it in the block
+                        const int sx = g4 >= 2 ? (se >> 16) & 15 : 2, sy = g4 >= 2 ? (se >> 20) & 15 : 2;
+                        unsigned wp = g4 == 0 ? 1u << A.cw : (unsigned)(lam - ma) << sx;
+                        unsigned wm = g4 == 0 ? 0u : (unsigned)ma << sy;
                         if (e >= E) wp = wm = 0;
                         const int iy = g4 >= 2 ? max(ec - 1, 0) : ec;
                         const int ix = g4 >= 2 ? (ctr ? iy : min(ec + 1, E - 1)) : ec;
@@ -843,7 +851,7 @@ __global__ void __launch_bounds__(DT, 2) k_plain_d64(PlainArgs<double> A) {
                         for (int g = 0; g < 4; ++g) {
                             const int at = (g * VI + i - c0) * CB + k;
                             const long long v = ((long long)Ch[at] << 32) + Cl[at] + (g == 0 ? z0 : 0);
-                            p[g] = bad ? NAN : (v == 0 ? 0.0 : mul2((double)v, g == 0 ? ek - A.cw : ek));
+                            p[g] = bad ? NAN : (v == 0 ? 0.0 : mul2((double)v, g == 0 ? ek - A.cw : ek - 2));
                         }
 #pragma unroll
                         for (int q = 0; q < 3; ++q) {
@@ -1230,13 +1238,7 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
     A.x = (T *)x;
     A.dxdr = (T *)dxdr;
     A.rdxdr = (T *)rdxdr;
-    // 2^vs >= |V| 2^row: |U| <= 1 and the row's power of two is within sqrt(2) of its factor
-    double bound = 2.0;
-    for (int m = 1; m <= t->twol / 2; ++m) bound *= (double)(t->twol - m + 1) / m;
-    A.vs = 0;
-    while (std::pow(4.0, A.vs) < bound) ++A.vs;
-    A.cw = 0;
-    while ((1 << A.cw) < t->twol) ++A.cw;
+    A.cw = t->p_cw;
     const int pass = plain_pass<T>(t, natoms);
     if (!work || work_bytes < SO4_WS_HEADER + plain_scratch<T>(t, natoms)) return SO4_ERR_WORKSPACE;
     const size_t tiles = (size_t)(pass + 31) / 32;

@@ -348,9 +348,21 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
         return c;
     };
     auto f_of = [&](int l, int m) { return std::sqrt(binom(l, m)); };
-    // the power of two nearest to f(l, mb): V and Z' as integers are scaled per row by it and
-    // its inverse, so that V's rows use the same range
-    auto row_exp = [&](int l, int mb) { return (int)std::lround(std::log2(f_of(l, mb))); };
+    // the power of two nearest to f(l, m), and to F(l, mb, ma): V and Z' as integers are scaled by
+    // it and its inverse, so that they use the range that U and Z do
+    auto f_exp = [&](int l, int m) { return (int)std::lround(std::log2(f_of(l, m))); };
+    auto ent_exp = [&](int l, int e) { return f_exp(l, e / (l + 1)) - f_exp(l, e % (l + 1)); };
+    // W = (l - m) Z'[m+1] -+ m Z'[m-1] on these scales, with two more bits for the neighbours'
+    // smaller ones; 2^p_cw bounds its weights
+    double wmax = 1.0;
+    for (int l = 1; l < ld; ++l)
+        for (int m = 0; m <= l; ++m) {
+            double w = (m < l) ? std::ldexp(l - m, f_exp(l, m) - f_exp(l, m + 1)) : 0.0;
+            if (m > 0) w += std::ldexp(m, f_exp(l, m) - f_exp(l, m - 1));
+            wmax = std::max(wmax, std::max(w, (double)l));
+        }
+    t->p_cw = 2;
+    while (std::ldexp(1.0, t->p_cw - 2) < wmax) ++t->p_cw;
     int prc = SO4_OK;
     std::vector<int> pblk_of(t->n_blk, -1), p_zof, p_bblk(t->n_b), p_sent, p_zent;
     std::vector<int4> p_blk, p_lam(ld), pz_unit, p_vent(nh), p_kblk(t->n_b, make_int4(0, 0, 0, 0));
@@ -374,14 +386,17 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
             pblk_of[bi] = (int)p_blk.size();
             p_blk.push_back(make_int4(bk.role_k[0], pz, E, lam));
             p_fac.push_back(f);
-            for (int e = 0; e < E; ++e) p_zent.push_back(pblk_of[bi] | (row_exp(lam, e / (lam + 1)) << 16));
+            for (int e = 0; e < E; ++e) p_zent.push_back(pblk_of[bi] | ((64 + ent_exp(lam, e)) << 16));
             p_zof.push_back(pz);
             pz += E;
         }
         p_lam[lam] = make_int4(E, first, (int)p_blk.size() - first, (int)p_sent.size());
         for (int e = 0; e < E; ++e) {
             const int ma = e % (lam + 1), mb = e / (lam + 1);
-            p_sent.push_back(ma | ((2 * mb == lam && 2 * ma == lam) ? 1 << 8 : 0) | (row_exp(lam, mb) << 16));
+            const int up = ma < lam ? 2 + f_exp(lam, ma) - f_exp(lam, ma + 1) : 2;
+            const int dn = ma > 0 ? 2 + f_exp(lam, ma) - f_exp(lam, ma - 1) : 2;
+            if (up < 0 || dn < 0) prc = SO4_ERR_UNSUPPORTED;  // f grows at most fourfold a step up to twol 16
+            p_sent.push_back(ma | ((2 * mb == lam && 2 * ma == lam) ? 1 << 8 : 0) | (up << 16) | (dn << 20));
         }
     }
     p_zof.push_back(pz);
@@ -428,11 +443,11 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     // U entry (l, mb, ma) = conj(a) P[ma] - conj(b) P[ma - 1], P row mb of level l - 1, or its
     // mirror (-1)^(..) conj of row l - 1 - mb: {index of P[ma], of P[ma - 1] (-1: none),
     // 1 conjugate | 2 negate P[ma] | 4 negate P[ma - 1], 1 middle-row centre | 2 ma = mb | l << 8 |
-    // row exponent << 16}
+    // 64 + exponent << 16}
     for (int l = 0; l < ld; ++l)
         for (int mb = 0; 2 * mb <= l; ++mb)
             for (int ma = 0; ma <= l; ++ma) {
-                int4 e = make_int4(-1, -1, 0, ((2 * mb == l && 2 * ma == l) ? 1 : 0) | (ma == mb ? 2 : 0) | (l << 8) | (row_exp(l, mb) << 16));
+                int4 e = make_int4(-1, -1, 0, ((2 * mb == l && 2 * ma == l) ? 1 : 0) | (ma == mb ? 2 : 0) | (l << 8) | ((64 + f_exp(l, mb) - f_exp(l, ma)) << 16));
                 const int L = l - 1;
                 if (l > 0 && 2 * mb <= L) {
                     if (ma < l) e.x = t->h_block[L] + mb * l + ma;
