@@ -99,8 +99,9 @@ __global__ void __launch_bounds__(NWF * 32) k_utot32(FwdArgs A) {
 // last two chains).  Each lane accumulates w_j sfac U over its images for its chain's rows;
 // the image groups are then added through shared memory in group order, the self term
 // f_c(0) w_site is put on the diagonal and u_norm applied (SO4.py:1480-1505, 560-597).
+// Twenty warps per SM up to twol 6 (sixteen above, where the registers end): lmax 3, 38,912 atoms 97 -> 87 us.
 template <int TWOL, int NW>
-__global__ void __launch_bounds__(NW * 32, (TWOL <= 8) ? 16 / NW : 1) k_utot_rc(FwdArgs A) {
+__global__ void __launch_bounds__(NW * 32, (TWOL <= 6) ? 20 / NW : ((TWOL <= 8) ? 16 / NW : 1)) k_utot_rc(FwdArgs A) {
     using UL = UtotLanes<TWOL>;
     constexpr int W = TWOL + 1, NACC = acc_block(TWOL + 1);
     extern __shared__ __align__(16) float ut_smem[];  // [NW][32][2 * NACC]
@@ -846,7 +847,7 @@ __global__ void __launch_bounds__(NWD * 32) k_deidrj(DArgs A) {
 // U rows are kept in shared memory by the forward sweep; one backward sweep of Y
 // gives the gradients with respect to conj(a), conj(b).
 template <int TWOL, int NT>
-__global__ void __launch_bounds__(NT, (TWOL <= 8) ? 512 / NT : 1) k_deidrj_rev(DArgs A, int64_t nimg) {
+__global__ void __launch_bounds__(NT, (TWOL <= 5) ? 640 / NT : ((TWOL <= 8) ? 512 / NT : 1)) k_deidrj_rev(DArgs A, int64_t nimg) {
     using RC = RowChain<TWOL>;
     constexpr int W = TWOL + 1;
     constexpr int NIT = 32 / RC::IPW, PASS = NIT * RC::IPW;  // images per warp: one per lane
@@ -960,7 +961,7 @@ __global__ void __launch_bounds__(NT, (TWOL <= 8) ? 512 / NT : 1) k_deidrj_rev(D
 // k_deidrj_rev with two lanes per image (so4_rev2.cuh): a warp takes 32 images, one per lane
 // for the set-up as above, then two iterations of 16 images, lane = 2 image + role.
 template <int TWOL, int NT>
-__global__ void __launch_bounds__(NT, (TWOL == 8) ? 3 : 2) k_deidrj_rev2(DArgs A, int64_t nimg) {
+__global__ void __launch_bounds__(NT, (TWOL == 8) ? 3 : 512 / NT) k_deidrj_rev2(DArgs A, int64_t nimg) {
     using Y = rev2::Layout<TWOL>;
     constexpr int W = TWOL + 1, NS = Y::NS;
     constexpr int IPI = 16, PASS = 32;  // images per iteration (two lanes each) and per warp
@@ -1094,17 +1095,22 @@ int launch_deidrj_rev_nt(const DArgs &D, int64_t nimg, cudaStream_t st) {
     return so4_launch_pdl(k_deidrj_rev<TWOL, NT>, dim3((unsigned)blocks), dim3(NT), smem, st, D, nimg);
 }
 
-// nt: threads per CTA, from the tables' tuning (256 up to twol 8, 128 above; both for twol 6, 8);
-// pair: two lanes per image (k_deidrj_rev2, twol 6 and 8: 256 threads at twol 6 with two
-// CTAs per SM, 128 at 8 with three) instead of one lane per row chain
+// nt: threads per CTA, from the tables' tuning (128 up to twol 5, with five CTAs per SM in 102
+// registers: 38,912 atoms of lmax 2 124 -> 108 us, of lmax 2.5 140 -> 126, two of 256 before; 256 for
+// twol 6 to 8, 128 above; both for twol 6, 8).  pair: two lanes per image (k_deidrj_rev2, twol 6 and
+// 8) instead of one lane per row chain; sixteen warps per SM at twol 6, by four CTAs where there are
+// many images (64,000 atoms 240 -> 230 us, 38,912 145 -> 140), by two below (4,096 atoms 18.5 us, by
+// four 19.3; 9,728, with 272,084 images, 37.3 and 37.6); three CTAs of 128 threads at twol 8.
+constexpr int64_t REV2_MANY = 400000;
 template <int TWOL>
 int launch_deidrj_rev(const DArgs &D, int64_t nimg, int nt, int pair, cudaStream_t st) {
     if constexpr (TWOL == 6 || TWOL == 8) {
-        if (pair) return launch_deidrj_rev2<TWOL, (TWOL == 6) ? 256 : 128>(D, nimg, st);
+        if (pair && TWOL == 6 && nimg <= REV2_MANY) return launch_deidrj_rev2<TWOL, (TWOL == 6) ? 256 : 128>(D, nimg, st);
+        if (pair) return launch_deidrj_rev2<TWOL, 128>(D, nimg, st);
         if (nt == 128) return launch_deidrj_rev_nt<TWOL, 128>(D, nimg, st);
         return launch_deidrj_rev_nt<TWOL, 256>(D, nimg, st);
     }
-    return launch_deidrj_rev_nt<TWOL, (TWOL <= 8) ? 256 : 128>(D, nimg, st);
+    return launch_deidrj_rev_nt<TWOL, (TWOL <= 5) ? 128 : ((TWOL <= 8) ? 256 : 128)>(D, nimg, st);
 }
 
 

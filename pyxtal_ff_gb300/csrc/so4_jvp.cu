@@ -33,8 +33,10 @@ struct JArgs {
 };
 
 // tangent of U_tot, one warp per centre (same lanes as k_utot_rc: UtotLanes)
+// Sixteen warps per SM up to twol 6, twelve at 7 and 8: 38,912 atoms of lmax 2.5 155 -> 132 us, of
+// lmax 3 (44 bytes of spills) 214 -> 201.  (At lmax 4 sixteen would spill 384 bytes.)
 template <int TWOL, int NW>
-__global__ void __launch_bounds__(NW * 32, (TWOL <= 4) ? 4 : ((TWOL <= 8) ? 3 : 1)) k_jvp_du_rc(JArgs A) {
+__global__ void __launch_bounds__(NW * 32, (TWOL <= 6) ? 4 : ((TWOL <= 8) ? 3 : 1)) k_jvp_du_rc(JArgs A) {
     using UL = UtotLanes<TWOL>;
     constexpr int W = TWOL + 1, NACC = acc_block(TWOL + 1);
     extern __shared__ __align__(16) float jv_smem[];
