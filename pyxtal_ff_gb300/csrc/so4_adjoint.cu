@@ -62,11 +62,10 @@ int set_smem(K kern, size_t smem) {
 struct FwdArgs {
     so4_params prm;
     float psi_fac, rc32;  // rfac0 pi / rcut and rcut in FP32, set on the host
-    int natoms, nh, nu, nz, nB;
+    int natoms, nh, nu, nB;
     const double *w_nb, *w_site, *img_r;
     const int32_t *img_ptr, *img_j;
-    const float *cg, *rootpq;
-    const BEnt *bent;
+    const float *rootpq;
     SmallTables st;
     const int4 *hmap;  // per half entry: accumulator slot, row, diagonal flag, u_norm F, u_norm
     float *utot, *x;
@@ -213,7 +212,6 @@ struct ZLArgs {
     const float2 *utot;
     const int2 *hfull;
     const int4 *unit, *seg;
-    const BEnt *bent;
     const ZBlk *blk;
     const int4 *blk_rk;    // per block: role components (so4_tables: d_blk_rk)
     const float4 *blk_rf;  // per block: role factors
@@ -1309,7 +1307,6 @@ static ZLArgs zl_args(const so4_tables *t, int natoms) {
     Z.nB = t->n_b;
     Z.nblk = t->n_blk;
     Z.hfull = t->d_hfull;
-    Z.bent = t->d_b;
     Z.blk = t->d_blk;
     Z.blk_rk = t->d_blk_rk;
     Z.blk_rf = t->d_blk_rf;
@@ -1447,16 +1444,13 @@ extern "C" int so4_forward32(const so4_tables *t, const so4_params *p, int natom
     A.natoms = natoms;
     A.nh = t->n_half;
     A.nu = t->n_u;
-    A.nz = t->n_z;
     A.nB = t->n_b;
     A.w_nb = d_w_nb;
     A.w_site = d_w_site;
     A.img_r = d_img_r;
     A.img_ptr = d_img_ptr;
     A.img_j = d_img_j;
-    A.cg = t->d_cg32;
     A.rootpq = t->d_rootpq32;
-    A.bent = t->d_b;
     fill_small_tables(t, A.st);
     A.hmap = t->d_hmap;
     A.utot = d_utot;
@@ -1761,16 +1755,13 @@ extern "C" int so4_utot32(const so4_tables *t, const so4_params *p, int natoms, 
     A.natoms = natoms;
     A.nh = t->n_half;
     A.nu = t->n_u;
-    A.nz = t->n_z;
     A.nB = t->n_b;
     A.w_nb = d_w_nb;
     A.w_site = d_w_site;
     A.img_r = d_img_r;
     A.img_ptr = d_img_ptr;
     A.img_j = d_img_j;
-    A.cg = t->d_cg32;
     A.rootpq = t->d_rootpq32;
-    A.bent = t->d_b;
     fill_small_tables(t, A.st);
     A.hmap = t->d_hmap;
     A.utot = d_utot;

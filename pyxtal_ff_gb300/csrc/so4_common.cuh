@@ -43,11 +43,6 @@ __device__ __forceinline__ cx<T> cmul(cx<T> a, cx<T> b) {
 template <typename T>
 __device__ __forceinline__ cx<T> cscale(cx<T> a, T s) { return mk<T>(a.re * s, a.im * s); }
 // acc += a * b
-template <typename T>
-__device__ __forceinline__ void cfma(cx<T> &acc, cx<T> a, cx<T> b) {
-    acc.re += a.re * b.re - a.im * b.im;
-    acc.im += a.re * b.im + a.im * b.re;
-}
 // Re(conj(a) * b)
 template <typename T>
 __device__ __forceinline__ T redot(cx<T> a, cx<T> b) { return a.re * b.re + a.im * b.im; }
@@ -85,9 +80,7 @@ struct so4_tables {
     std::vector<int> h_block;  // ldim + 1
     std::vector<double> unorm_l;  // per level
     // device copies
-    float *d_cg32 = nullptr;
     float *d_rootpq32 = nullptr;
-    BEnt *d_b = nullptr;
     ZBlk *d_blk = nullptr;
     // per Z block, packed for the window kernels' coefficient loop: the components of its
     // roles {k0, k1, k2, nrole} (missing roles repeat k0) and their FP32 factors (0 when missing)
@@ -402,18 +395,6 @@ __device__ void warp_uarray(const SmallTables &st, const T *rootpq, const CK<T> 
             __syncwarp();
         }
     }
-}
-
-// acc += a b and acc -= a b on complex values, as four FMAs each.
-template <typename T>
-__device__ __forceinline__ void cmac(cx<T> &acc, const cx<T> &a, const cx<T> &b) {
-    acc.re = fma(a.re, b.re, fma(-a.im, b.im, acc.re));
-    acc.im = fma(a.re, b.im, fma(a.im, b.re, acc.im));
-}
-template <typename T>
-__device__ __forceinline__ void cmsub(cx<T> &acc, const cx<T> &a, const cx<T> &b) {
-    acc.re = fma(-a.re, b.re, fma(a.im, b.im, acc.re));
-    acc.im = fma(-a.re, b.im, fma(-a.im, b.re, acc.im));
 }
 
 // Number of half-layout entries one dB/dr section of level lam sums over

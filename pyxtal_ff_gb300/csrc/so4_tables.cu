@@ -81,9 +81,7 @@ int upload(T **dst, const std::vector<T> &src) {
 }
 
 void free_device(so4_tables *t) {
-    cudaFree(t->d_cg32);
     cudaFree(t->d_rootpq32);
-    cudaFree(t->d_b);
     cudaFree(t->d_blk);
     cudaFree(t->d_blk_rk);
     cudaFree(t->d_blk_rf);
@@ -568,7 +566,6 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     std::vector<float> rp32(ld * ld, 0.f);
     for (int p = 1; p < ld; ++p)
         for (int q = 1; q < ld; ++q) rp32[p * ld + q] = (float)std::sqrt((double)p / (double)q);
-    std::vector<float> cg32(t->cglist.begin(), t->cglist.end());
     // B component of each block (blocks with l >= l1)
     std::vector<int> blk_k(t->n_blk, -1);
     for (int k = 0; k < t->n_b; ++k)
@@ -869,9 +866,7 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     if (!rc) rc = upload(&t->d_jbase, jbase);
     if (!rc) rc = upload(&t->d_jfac, jfac);
     if (!rc) rc = upload(&t->d_wca, wca);
-    if (!rc) rc = upload(&t->d_cg32, cg32);
     if (!rc) rc = upload(&t->d_rootpq32, rp32);
-    if (!rc) rc = upload(&t->d_b, bent);
     if (!rc) rc = upload(&t->d_pz_unit, pz_unit);
     if (!rc) rc = upload(&t->d_p_vent, p_vent);
     if (!rc) rc = upload(&t->d_p_lam, p_lam);
