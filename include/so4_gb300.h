@@ -47,7 +47,8 @@ enum so4_status {
     SO4_ERR_NO_NEIGHBOR = 7,  /* an atom has no neighbour image (reference raises ValueError, SO4.py:275) */
     SO4_ERR_REVERSE = 8,      /* an image has no reverse image (asymmetric list)    */
     SO4_ERR_TOO_LARGE = 9,    /* problem needs more than the fixed scratch of so4_adjoint32_noalloc */
-    SO4_ERR_SLOTS = 10        /* an atom has more images than the per-atom key slots of so4_nl_count_keys */
+    SO4_ERR_SLOTS = 10,       /* an atom has more images than the per-atom key slots of so4_nl_count_keys */
+    SO4_ERR_OFFSET = 11       /* status bit beside SO4_ERR_CAPACITY: an image more than 511 cells away */
 };
 
 /* Maximum 2*lmax the kernels are compiled for (lmax <= 6). */
@@ -206,10 +207,11 @@ int so4_nl_sort(const so4_geom *d_geom, int nstruct, int nbins, const double *d_
  *   so4_nl_scan_range        d_img_ptr[a0 .. a1] = d_img_ptr[a0] (0 when a0 = 0) + the exclusive
  *                            scan of those counts: ranges are scanned in order, each after the
  *                            previous one's scan;
- *   so4_nl_sort_range        so4_nl_sort for the centres [a0, a1) without the pair counts, and,
- *                            if any capacity was exceeded so far, empties d_img_ptr[a0 .. a1]
- *                            so that work enqueued behind it on the range reads nothing out of
- *                            bounds.
+ *   so4_nl_sort_range        so4_nl_sort for the centres [a0, a1) without the pair counts.
+ *                            d_img_ptr[a0 .. a1] is bounded by nimg, and a centre whose images
+ *                            do not fit the arrays or its slots gets images beyond any cutoff
+ *                            in their place, so that work enqueued behind it on the range reads
+ *                            nothing out of bounds (and so4_nl_summary reports the overflow).
  * The lite reverse pass (so4_nl_pairs with NULL pair arrays) and so4_nl_summary run after
  * every range is sorted. */
 int so4_nl_bins(const so4_geom *d_geom, int nstruct, int nbins, const double *d_pos, const int *d_atom_struct,
@@ -224,7 +226,8 @@ int so4_nl_sort_range(const so4_geom *d_geom, int nstruct, int nbins, const doub
                       int32_t *d_img_off, double *d_img_r, void *d_work, size_t work_bytes, void *stream);
 
 /* {total images, total pairs, status bits} after the three passes (d_pair_ptr may
- * be NULL after pass 1 only), written to ((int *)d_work)[4..6]; with h_summary
+ * be NULL after pass 1 only; the images are those counted, also where the arrays
+ * hold fewer), written to ((int *)d_work)[4..6]; with h_summary
  * non-NULL also copied there by one synchronising read.  With h_summary NULL the
  * call does not synchronise (for stream capture); the caller reads the three
  * ints later, e.g. with the step's results.  When a capacity was exceeded (status

@@ -21,6 +21,7 @@ SO4_ERR_NO_NEIGHBOR = 7
 SO4_ERR_REVERSE = 8
 SO4_ERR_TOO_LARGE = 9
 SO4_ERR_SLOTS = 10
+SO4_ERR_OFFSET = 11
 
 _MESSAGES = {
     SO4_ERR_ARG: "invalid argument",
@@ -33,6 +34,7 @@ _MESSAGES = {
     SO4_ERR_REVERSE: "neighbour list is not symmetric",
     SO4_ERR_TOO_LARGE: "problem exceeds the fixed 64 MiB scratch of so4_adjoint32_noalloc",
     SO4_ERR_SLOTS: "an atom has more images than the per-atom key slots",
+    SO4_ERR_OFFSET: "an image offset is beyond the encodable 511 cells",
 }
 
 

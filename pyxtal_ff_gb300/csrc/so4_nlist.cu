@@ -21,6 +21,9 @@ namespace {
 
 constexpr int OFF_BIAS = 512;  // image offsets are packed in 10 bits each
 constexpr int OFF_MAX = 511;
+// words of the workspace header after the status: the list's totals as so4_nl_summary leaves them
+// (4 .. 6), the largest count of an atom, and the images counted so far
+constexpr int HDR_SUMMARY = 4, HDR_MAX_COUNT = 8, HDR_IMAGES = 9;
 
 struct NLWork {
     int *status;
@@ -144,12 +147,15 @@ __global__ void k_bin_fill(const int *astruct, int natoms, NLWork w) {
 // thread, coalesced), warp-shuffle scans inside, a running carry across chunks; the next
 // chunk's values are loaded before the current one is scanned.  With chained != 0 the scan
 // continues a previous one: out[0] already holds the running total before in[0] (ranges of
-// centres scanned one after another).
-__global__ void __launch_bounds__(1024) k_scan(const int *in, int *out, int n, int chained = 0) {
+// centres scanned one after another) and is not written again, work on the range before it may
+// have bounded it.  total, if given, counts the values of all ranges on its own: what the arrays'
+// capacity does to out does not reach it.
+__global__ void __launch_bounds__(1024) k_scan(const int *in, int *out, int n, int chained = 0, int *total = nullptr) {
     __shared__ int wsum[32];
     __shared__ int carry_s;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    if (t == 0) carry_s = chained ? out[0] : 0;
+    int first = 0;
+    if (t == 0) carry_s = first = chained ? out[0] : 0;
     int nv[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) nv[q] = (4 * t + q < n) ? __ldg(in + 4 * t + q) : 0;
@@ -186,14 +192,17 @@ __global__ void __launch_bounds__(1024) k_scan(const int *in, int *out, int n, i
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int i = base + 4 * t + q;
-            if (i < n) out[i] = run;
+            if (i < n && (i > 0 || !chained)) out[i] = run;
             run += v[q];
         }
         __syncthreads();
         if (t == 1023) carry_s = run;
         __syncthreads();
     }
-    if (t == 0) out[n] = carry_s;
+    if (t == 0) {
+        out[n] = carry_s;
+        if (total) *total = (chained ? *total : 0) + carry_s - first;
+    }
 }
 
 // The bins of a small list (natoms <= BIN_ATOMS, nbins <= BIN_BINS) by one CTA: header cleared,
@@ -261,14 +270,15 @@ __global__ void k_set_int(int *p, int v) { *p = v; }
 
 // {images, pairs, status bits}, and then, if a capacity was exceeded (or an offset did not
 // fit), every image and pair range emptied, so that kernels enqueued behind the list without
-// a host check (a captured step) read nothing out of bounds.  The thread of the last entry
-// takes the totals before it empties its own entry.
+// a host check (a captured step) read nothing out of bounds.  The images are the scan's own
+// total: img_ptr may have been bounded by k_clamp_range.  The thread of the last entry takes the
+// pairs before it empties its own entry.
 __global__ void k_summary(int32_t *img_ptr, int32_t *pair_ptr, int natoms, const int *status, int *out) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > natoms) return;
     const int bits = *status;
     if (i == natoms) {
-        out[0] = natoms > 0 ? img_ptr[natoms] : 0;
+        out[0] = natoms > 0 ? status[HDR_IMAGES] : 0;
         out[1] = (natoms > 0 && pair_ptr) ? pair_ptr[natoms] : 0;
         out[2] = bits;
     }
@@ -277,12 +287,12 @@ __global__ void k_summary(int32_t *img_ptr, int32_t *pair_ptr, int natoms, const
     if (pair_ptr) pair_ptr[i] = 0;
 }
 
-// The emptying for a range: after a range's sort, if any capacity was exceeded so far, empty
-// the range's image ranges (img_ptr[a0 .. a1]) before work on them is enqueued.
-__global__ void k_clamp_range(int32_t *img_ptr, int a0, int a1, const int *status) {
+// After a range's sort, img_ptr[a0 .. a1] bounded by the arrays' capacity before work on the range
+// is enqueued.  Neighbouring ranges share a boundary entry while both are at work: whichever of them
+// bounds it, it gets the same value, and stays in order with the entries around it.
+__global__ void k_clamp_range(int32_t *img_ptr, int a0, int a1, int64_t cap) {
     const int i = a0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > a1 || !(*(volatile const int *)status & (1 << SO4_ERR_CAPACITY))) return;
-    img_ptr[i] = 0;
+    if (i <= a1 && img_ptr[i] > cap) img_ptr[i] = (int32_t)cap;
 }
 
 // One warp per centre.  MODE 0: count images into w.cnt.  MODE 1: write the
@@ -378,6 +388,7 @@ __global__ void __launch_bounds__(256) k_scan_images(const so4_geom *geom, const
                 }
                 if (MODE >= 1) {
                     if (abs(o[0]) > OFF_MAX || abs(o[1]) > OFF_MAX || abs(o[2]) > OFF_MAX) {
+                        flag(w.status, SO4_ERR_OFFSET);
                         flag(w.status, SO4_ERR_CAPACITY);
                         continue;
                     }
@@ -414,7 +425,7 @@ __global__ void __launch_bounds__(256) k_scan_images(const so4_geom *geom, const
         const int tot = (PARTS > 1) ? s_cnt[wc] : mine;
         w.cnt[a] = tot;
         if (tot == 0) flag(w.status, SO4_ERR_NO_NEIGHBOR);
-        if (MODE == 2) atomicMax(w.status + 8, tot);
+        if (MODE == 2) atomicMax(w.status + HDR_MAX_COUNT, tot);
     }
 }
 
@@ -430,6 +441,8 @@ void launch_scan(const so4_geom *geom, const double *pos, const int *astruct, do
     so4_count_launch();
 }
 
+constexpr double FAR_AWAY = 1e6;  // A
+
 // One warp per centre: rank-sort the keys, write the sorted images and count pairs.
 __global__ void k_sort(const so4_geom *geom, const double *pos, const int *astruct, int natoms,
                        const int32_t *img_ptr, int32_t *img_j, int32_t *img_off, double *img_r, NLWork w,
@@ -441,10 +454,17 @@ __global__ void k_sort(const so4_geom *geom, const double *pos, const int *astru
     const so4_geom &g = geom[astruct[a]];
     const int p0 = img_ptr[a], p1 = img_ptr[a + 1];
     if (p1 > w.cap_img || (w.slot_cap > 0 && p1 - p0 > w.slot_cap)) {
-        // the arrays (or this atom's key slots) are too small for this call; the host grows them
+        // the arrays (or this atom's key slots) are too small for this call; the host grows them.
+        // Work enqueued on a range reads its entries all the same: images beyond any cutoff.
         if (lane == 0) {
             w.cnt[a] = 1;
             flag(w.status, SO4_ERR_CAPACITY);
+        }
+        for (int64_t q = p0 + lane; q < p1 && q < w.cap_img; q += 32) {
+            img_j[q] = a;
+            img_off[3 * q] = img_off[3 * q + 1] = img_off[3 * q + 2] = 0;
+            img_r[3 * q] = FAR_AWAY;
+            img_r[3 * q + 1] = img_r[3 * q + 2] = 0.0;
         }
         return;
     }
@@ -754,7 +774,7 @@ extern "C" int so4_nl_count(const so4_geom *d_geom, int nstruct, int nbins, cons
     const int rc = make_bins(w, d_geom, nbins, d_pos, d_astruct, natoms, st);
     if (rc) return rc;
     launch_scan<0>(d_geom, d_pos, d_astruct, rcut, nullptr, w, 0, natoms, st);
-    k_scan<<<1, 1024, 0, st>>>(w.cnt, d_img_ptr, natoms);
+    k_scan<<<1, 1024, 0, st>>>(w.cnt, d_img_ptr, natoms, 0, w.status + HDR_IMAGES);
     so4_count_launch();
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
 }
@@ -841,7 +861,7 @@ extern "C" int so4_nl_scan_range(int natoms, int nbins, int slot_cap, int a0, in
         }
         return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
     }
-    k_scan<<<1, 1024, 0, st>>>(w.cnt + a0, d_img_ptr + a0, a1 - a0, a0 > 0 ? 1 : 0);
+    k_scan<<<1, 1024, 0, st>>>(w.cnt + a0, d_img_ptr + a0, a1 - a0, a0 > 0 ? 1 : 0, w.status + HDR_IMAGES);
     so4_count_launch();
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
 }
@@ -874,7 +894,7 @@ extern "C" int so4_nl_sort_range(const so4_geom *d_geom, int nstruct, int nbins,
     k_sort<<<(a1 - a0 + warps - 1) / warps, 32 * warps, 0, st>>>(d_geom, d_pos, d_astruct, a1, d_img_ptr, d_img_j,
                                                                  d_img_off, d_img_r, w, a0);
     so4_count_launch();
-    k_clamp_range<<<(a1 - a0 + 1 + 255) / 256, 256, 0, st>>>(d_img_ptr, a0, a1, w.status);
+    k_clamp_range<<<(a1 - a0 + 1 + 255) / 256, 256, 0, st>>>(d_img_ptr, a0, a1, w.cap_img);
     so4_count_launch();
     return cudaGetLastError() == cudaSuccess ? SO4_OK : SO4_ERR_CUDA;
 }
@@ -960,7 +980,7 @@ extern "C" int so4_nl_summary(const int32_t *d_img_ptr, const int32_t *d_pair_pt
                               size_t work_bytes, void *stream, int *h_summary) {
     if (!d_work || work_bytes < SO4_WS_HEADER || natoms < 0) return SO4_ERR_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    int *dev = (int *)d_work + 4;  // header scratch after the status word
+    int *dev = (int *)d_work + HDR_SUMMARY;
     k_summary<<<(natoms + 256) / 256, 256, 0, st>>>((int32_t *)d_img_ptr, (int32_t *)d_pair_ptr, natoms,
                                                     (const int *)d_work, dev);
     so4_count_launch();

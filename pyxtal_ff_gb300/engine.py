@@ -315,9 +315,12 @@ def check_summary(M, P, bits, cap_m=None, cap_p=None):
         return False
     if bits & (1 << _lib.SO4_ERR_NONFINITE):
         raise ValueError("positions contain NaN or Inf")
-    for code in (_lib.SO4_ERR_CAPACITY, _lib.SO4_ERR_REVERSE):  # capacity here: an image offset beyond 511 cells
-        if bits & (1 << code):
-            raise _lib.SO4Error(code, "neighbour list")
+    if bits & (1 << _lib.SO4_ERR_OFFSET):
+        raise _lib.SO4Error(_lib.SO4_ERR_CAPACITY, "neighbour list: an image more than 511 cells away")
+    if bits & (1 << _lib.SO4_ERR_CAPACITY):
+        return False
+    if bits & (1 << _lib.SO4_ERR_REVERSE):
+        raise _lib.SO4Error(_lib.SO4_ERR_REVERSE, "neighbour list")
     return True
 
 
