@@ -27,6 +27,7 @@ from __future__ import annotations
 import numpy as np
 
 from .nn import EV2GPA, NeuralNetworkPotential
+from .structures import pbc_of
 
 # ASE's GPa in eV/A^3 (CODATA 2014, ASE's default): 1 / 160.21766208
 ASE_GPA = 1.0 / 160.21766208
@@ -65,6 +66,19 @@ def compute_descriptor(function, structure):
     return _descriptor_object(function).calculate(structure, stress_per_atom=True)
 
 
+def _settings(function):
+    """What the descriptor is built from, as values that can be compared later."""
+    p, w = function["parameters"], function.get("weights")
+    return (function["type"], p["lmax"], function["Rc"], function["cutoff"], p.get("normalize_U", False),
+            p.get("rfac", 0.99363), tuple(sorted(w.items())) if isinstance(w, dict) else w)
+
+
+def _networks(model):
+    """A model and its networks, to be held and compared by identity."""
+    nets = getattr(model, "models", None)
+    return (model, *nets.values()) if isinstance(nets, dict) else (model,)
+
+
 def _element_order(symbols, elements):
     """The atoms element after element, as the networks' energies are stored."""
     symbols = np.asarray(symbols)
@@ -84,7 +98,7 @@ class PyXtalFFCalculator:
         self.results = {}
         self.atoms = None
         self._atoms_obj = None
-        self._calc = None
+        self._calc, self._calc_settings, self._used = None, None, None
         self._step, self._step_key, self._last_key, self._order = None, None, None, None
 
     def _ff(self):
@@ -97,10 +111,17 @@ class PyXtalFFCalculator:
 
     def _key(self, atoms):
         return (np.array(atoms.positions, dtype=np.float64).copy(), np.array(atoms.get_cell(), dtype=np.float64).copy(),
-                np.array(atoms.numbers).copy())
+                np.array(atoms.numbers).copy(), pbc_of(atoms))
 
     def _changed(self, atoms):
         if self.atoms is None or not self.results:
+            return True
+        ff = self.parameters["ff"]
+        settings, models = self._used
+        if ff is None or settings != _settings(ff._descriptors):
+            return True
+        now = _networks(ff.model)
+        if len(now) != len(models) or any(a is not b for a, b in zip(now, models)):
             return True
         return any(a.shape != b.shape or not np.array_equal(a, b) for a, b in zip(self._key(atoms), self.atoms))
 
@@ -112,6 +133,9 @@ class PyXtalFFCalculator:
             raise NotImplementedError("route='adjoint' supports unit 'eV'")
         f = ff._descriptors
         p = f["parameters"]
+        settings = _settings(f)
+        if self._calc_settings not in (None, settings):  # another force field: nothing kept applies
+            self._calc, self._step, self._last_key = None, None, None
         if self._calc is None:
             kind = "SNAP" if f["type"] in ("SNAP", "snap") else "SO4"
             if f["type"] not in ("SNAP", "snap", "SO4", "Bispectrum", "bispectrum"):
@@ -119,12 +143,14 @@ class PyXtalFFCalculator:
             self._calc = SO4Calculator(lmax=p["lmax"], rcut=f["Rc"], kind=kind, weights=f.get("weights"),
                                        rfac0=p.get("rfac", 0.99363), cutoff_function=f["cutoff"],
                                        normalize_U=p.get("normalize_U", False))
+        self._calc_settings = settings
         # an MD or relaxation loop moves only the positions: from the second structure of one
-        # layout (cell, pbc, species, model) on, the step is one CUDA-graph replay
+        # layout (cell, pbc, species, model; the key holds the networks, so that another one cannot
+        # take a freed one's place) on, the step is one CUDA-graph replay
         # (SO4Calculator.capture), bit for bit the uncaptured compute()
         positions, cell, pbc, numbers, symbols = as_arrays(atoms)
-        key = (cell.tobytes(), pbc.tobytes(), numbers.tobytes(), symbols, id(ff.model), tuple(ff.model.elements),
-               tuple(id(ff.model.models[e]) for e in ff.model.elements))
+        key = (cell.tobytes(), pbc.tobytes(), numbers.tobytes(), symbols, tuple(ff.model.elements), ff.model,
+               tuple(ff.model.models[e] for e in ff.model.elements))
         if self._step is not None and self._step_key != key:
             self._step = None
         if self._step is None and self._last_key == key:
@@ -188,6 +214,7 @@ class PyXtalFFCalculator:
         else:
             self.results["stress"] = self.results["stress_zbl"] + self.results["stress_ml"]
         self.atoms = self._key(atoms)
+        self._used = (_settings(ff._descriptors), _networks(ff.model))
 
     def get_property(self, name, atoms=None):
         if atoms is not None and self._changed(atoms):

@@ -90,14 +90,19 @@ class Atoms:
         return Atoms(self.numbers.copy(), self.positions.copy(), self.cell.copy(), self.pbc.copy())
 
 
+def pbc_of(atoms):
+    """The three periodicity flags (int32) of an Atoms or an ase.Atoms."""
+    pbc = getattr(atoms, "pbc", True)
+    if callable(getattr(atoms, "get_pbc", None)):
+        pbc = atoms.get_pbc()
+    return np.array(np.broadcast_to(np.asarray(pbc, dtype=bool), (3,)), dtype=np.int32)
+
+
 def as_arrays(atoms):
     """(positions, cell, pbc, numbers, symbols) from an Atoms or an ase.Atoms."""
     pos = np.ascontiguousarray(np.asarray(atoms.positions, dtype=np.float64))
     cell = np.ascontiguousarray(np.asarray(atoms.get_cell(), dtype=np.float64).reshape(3, 3))
-    pbc = getattr(atoms, "pbc", True)
-    if callable(getattr(atoms, "get_pbc", None)):
-        pbc = atoms.get_pbc()
-    pbc = np.array(np.broadcast_to(np.asarray(pbc, dtype=bool), (3,)), dtype=np.int32)
+    pbc = pbc_of(atoms)
     numbers = np.asarray(atoms.numbers, dtype=np.int64)
     symbols = list(map(str, atoms.symbols))
     return pos, cell, pbc, numbers, symbols
