@@ -1746,6 +1746,13 @@ extern "C" size_t so4_linear_workspace_size(const so4_tables *t, int natoms, int
 extern "C" int so4_utot32(const so4_tables *t, const so4_params *p, int natoms, const double *d_w_nb,
                           const double *d_w_site, const int32_t *d_img_ptr, const int32_t *d_img_j,
                           const double *d_img_r, float *d_utot, void *stream) {
+    return so4_utot32_as(t, p, t ? t->d_hmap : nullptr, natoms, d_w_nb, d_w_site, d_img_ptr, d_img_j, d_img_r, d_utot,
+                         stream);
+}
+
+int so4_utot32_as(const so4_tables *t, const so4_params *p, const int4 *hmap, int natoms, const double *d_w_nb,
+                  const double *d_w_site, const int32_t *d_img_ptr, const int32_t *d_img_j, const double *d_img_r,
+                  float *d_utot, void *stream) {
     if (!t || !p || natoms < 0 || !d_utot) return SO4_ERR_ARG;
     if (p->twol != t->twol || !(p->rcut > 0.0) || !(p->rfac0 > 0.0)) return SO4_ERR_ARG;
     if (p->cutoff_id < 1 || p->cutoff_id > 7) return SO4_ERR_UNSUPPORTED;
@@ -1763,7 +1770,7 @@ extern "C" int so4_utot32(const so4_tables *t, const so4_params *p, int natoms, 
     A.img_j = d_img_j;
     A.rootpq = t->d_rootpq32;
     fill_small_tables(t, A.st);
-    A.hmap = t->d_hmap;
+    A.hmap = hmap;
     A.utot = d_utot;
     A.x = nullptr;
     A.psi_fac = (float)(p->rfac0 * SO4_PI / p->rcut);

@@ -94,6 +94,7 @@ struct so4_tables {
     // bits of u_norm[L] F, bits of u_norm[L], 0}: where the row-chain kernels keep it and how
     // it is finished (F the row scale of the scaled recursion, so4_tables.cu)
     int4 *d_hmap = nullptr;
+    int4 *d_hmap_v = nullptr;   // the same without F (the third word twice): the scaled rows V themselves
     float *d_yscale = nullptr;  // n_half: the row-scale F of each half entry (so4_tables.cu)
     // Plain path (so4_plain.cu).  Its arrays carry U in the scaled form V = U / F and Z as
     // F Z (F the row scale), each Z block cut to its dB/dr section, blocks ordered by level.
@@ -470,6 +471,11 @@ int so4_launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, c
 // device.  The attribute is set only when the limit grows, so launches after the
 // first make no runtime call besides the launch (safe inside stream capture).
 int so4_set_smem(const void *kern, size_t smem);
+// so4_utot32, each entry finished by the factor that hmap holds (t->d_hmap: U; t->d_hmap_v: V = U / F;
+// the same at twol 0 and 1, where F = 1).
+int so4_utot32_as(const so4_tables *t, const so4_params *p, const int4 *hmap, int natoms, const double *d_w_nb,
+                  const double *d_w_site, const int32_t *d_img_ptr, const int32_t *d_img_j, const double *d_img_r,
+                  float *d_utot, void *stream);
 // The JVP's Z contraction by the window kernel (so4_adjoint.cu): dB [natoms][nB] from
 // U_tot and its tangent dU (both [natoms][nh] float2), with n_jslot x natoms floats of
 // slot scratch.

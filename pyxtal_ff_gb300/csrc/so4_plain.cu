@@ -72,14 +72,13 @@ struct PlainArgs {
     const int *sent, *bblk, *zent, *wk;
     const int4 *wpos;
     const float4 *wfac;
-    const float *yscale;
     SmallTables st;
     int want_stress;
     T *x, *dxdr, *rdxdr;
     // scratch of this pass, centre c = a - a0 in tile c / 32, lane c % 32:
     pc<T> *ut;       // U_tot, full rows: [tile][n_u][32]
     pc<T> *zt;       // Z': [tile][32 / ZQ][n_z][ZQ]
-    float2 *uh;      // FP32: U_tot, half layout [centre][n_half]
+    float2 *uh;      // FP32: V_tot, half layout [centre][n_half]
     longlong2 *zi;   // k_plain_d64 without room for them in shared memory: integers [centre][n_z]
 };
 
@@ -130,6 +129,22 @@ __device__ __forceinline__ void plain_rows(const SmallTables &st, const int4 *__
     __syncthreads();
 }
 
+// conj(a) and conj(b) of an image (SO4.py:879-884): {cos psi, g z, g y, g x}, with g = sin psi / r, as
+// one rounded quotient (ir = 1 / r and a correction by its remainder), returned.  The rounding of
+// these four numbers, l times over at level l, is the largest error of U and dB/dr next to that of
+// psi: with sin psi (z (1 / r)) dB/dr was up to 1.2 times as far off (FP64, lmax 6, against 64-bit
+// mantissas: 2.24e-15 instead of 1.87e-15 in the 2-norm).  FP32 takes the quotient's remainder into
+// the products as well.
+template <typename T>
+__device__ __forceinline__ T cayley_klein(T sn, T cs, T x, T y, T z, T r, T ir, T (&ck)[4]) {
+    const T q = sn * ir, lo = fma(-q, r, sn) * ir, g = q + lo;
+    ck[0] = cs;
+    ck[1] = sizeof(T) == 8 ? g * z : fma(q, z, lo * z);
+    ck[2] = sizeof(T) == 8 ? g * y : fma(q, y, lo * y);
+    ck[3] = sizeof(T) == 8 ? g * x : fma(q, x, lo * x);
+    return g;
+}
+
 constexpr int UT = 256;  // threads of k_plain_u
 
 __global__ void __launch_bounds__(UT) k_plain_u(PlainArgs<double> A) {
@@ -164,12 +179,11 @@ __global__ void __launch_bounds__(UT) k_plain_u(PlainArgs<double> A) {
                 }
             }
             const double r = sqrt(x * x + y * y + z * z);
-            CK<double> k;
-            make_ck<double, false>(x, y, z, r, A.psi_fac * r, k);
-            ck[tid] = k.ca.re;
-            ck[32 + tid] = k.ca.im;
-            ck[64 + tid] = k.cb.re;
-            ck[96 + tid] = k.cb.im;
+            double sn, cs, k[4];
+            sincos(A.psi_fac * r, &sn, &cs);
+            cayley_klein<double>(sn, cs, x, y, z, r, 1.0 / r, k);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ck[32 * i + tid] = k[i];
             wsf[tid] = w;
         }
         __syncthreads();
@@ -180,12 +194,16 @@ __global__ void __launch_bounds__(UT) k_plain_u(PlainArgs<double> A) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int e = tid + q * UT;
+                double pr[2] = {0.0, 0.0}, pi[2] = {0.0, 0.0};  // even and odd images of this part
                 if (e < nh)
+#pragma unroll 2
                     for (int i = 0; i < nc; ++i) {
                         const pc<double> v = V[v_at(e, i)];
-                        ar[q] = fma(wsf[c0 + i], v.re, ar[q]);
-                        ai[q] = fma(wsf[c0 + i], v.im, ai[q]);
+                        pr[i & 1] = fma(wsf[c0 + i], v.re, pr[i & 1]);
+                        pi[i & 1] = fma(wsf[c0 + i], v.im, pi[i & 1]);
                     }
+                ar[q] += pr[0] + pr[1];
+                ai[q] += pi[0] + pi[1];
             }
             __syncthreads();
         }
@@ -213,8 +231,9 @@ __global__ void __launch_bounds__(UT) k_plain_u(PlainArgs<double> A) {
     }
 }
 
-// FP32: the tiles of 32 centres from the row-chain kernel's U_tot (so4_utot32), divided by the
-// row scale F; a CTA per tile, lane = centre within a warp.
+// FP32: the tiles of 32 centres from the row-chain kernel's sums, which are V already (U divided by F
+// here took two more roundings: x at lmax 4 2.84e-7 off instead of 2.5e-7); a CTA per tile, lane =
+// centre within a warp.
 __global__ void __launch_bounds__(256) k_plain_tile(PlainArgs<float> A) {
     __shared__ float2 s[32 * 33];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, c0 = blockIdx.x * 32, nh = A.n_half;
@@ -226,9 +245,8 @@ __global__ void __launch_bounds__(256) k_plain_tile(PlainArgs<float> A) {
             if (e0 + lane < nh) s[lane * 33 + c] = A.uh[(size_t)(c0 + c) * nh + e0 + lane];
         __syncthreads();
         for (int i = wid; i < 32 && e0 + i < nh; i += 8) {
-            const float f = 1.f / __ldg(A.yscale + e0 + i);
             const float2 u = lane < live ? s[i * 33 + lane] : make_float2(0.f, 0.f);
-            pc<float> v = {u.x * f, u.y * f};
+            pc<float> v = {u.x, u.y};
             const int2 m = __ldg(A.hfull + e0 + i);
             ut[(size_t)m.x * 32] = v;
             if (m.y >= 0) {
@@ -365,13 +383,19 @@ __global__ void __launch_bounds__(256) k_plain_b(PlainArgs<T> A) {
     const int lam = b.w, cnt = b.z;
     const pc<T> *u = A.ut + ((size_t)blockIdx.x * A.n_u + A.st.u_block[lam]) * 32 + lane;
     const pc<T> *z = plain_zt(A, blockIdx.x * 32 + lane) + (size_t)b.y * ZQ<T>;
-    T s = T(0);
+    // four sums side by side: half the rounding of one of up to 49 terms (x at lmax 6 5.6e-16
+    // instead of 6.0e-16 off)
+    T s4[4] = {T(0), T(0), T(0), T(0)};
     const int full = (lam & 1) ? cnt : cnt - 1;
-#pragma unroll 4
-    for (int e = 0; e < full; ++e) {
-        const pc<T> p = u[(size_t)e * 32], q = z[(size_t)e * ZQ<T>];
-        s = fma(p.re, q.re, fma(p.im, q.im, s));
+    for (int e = 0; e < full; e += 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (e + i < full) {
+                const pc<T> p = u[(size_t)(e + i) * 32], q = z[(size_t)(e + i) * ZQ<T>];
+                s4[i] = fma(p.re, q.re, fma(p.im, q.im, s4[i]));
+            }
     }
+    T s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
     if (full < cnt) {
         const pc<T> p = u[(size_t)full * 32], q = z[(size_t)full * ZQ<T>];
         s += T(0.5) * (p.re * q.re + p.im * q.im);
@@ -413,6 +437,8 @@ __device__ __forceinline__ void plain_image(const PlainArgs<T> &A, int a, int m,
     }
     T sf, dsf, sn, cs;
     cutoff_fn<T>(A.prm.cutoff_id, r, A.rc, sf, dsf);
+    // psi as the U_tot kernels round it: its error moves U and dU/dr alike, and most of it cancels (with
+    // what it lost put back in here alone FP32 dB/dr at lmax 6 was 1.4e-6 off instead of 1.1e-6)
     if (sizeof(T) == 8) {
         double s_, c_;
         sincos((double)(A.psi_fac * r), &s_, &c_);
@@ -424,12 +450,14 @@ __device__ __forceinline__ void plain_image(const PlainArgs<T> &A, int a, int m,
         sn = (T)s_;
         cs = (T)c_;
     }
-    const T ir = T(1) / r, n[3] = {x * ir, y * ir, z * ir};
-    ck[0] = cs;
-    ck[1] = sn * n[2];
-    ck[2] = sn * n[1];
-    ck[3] = sn * n[0];
-    const T ws = w * sf, wd = w * dsf, sr = sn * ir;
+    const T ir = T(1) / r;
+    auto unit = [&](T v) {  // v / r, rounded once
+        const T q = v * ir;
+        return fma(fma(-q, r, v), ir, q);
+    };
+    const T n[3] = {unit(x), unit(y), unit(z)};
+    const T sr = cayley_klein<T>(sn, cs, x, y, z, r, ir, ck);
+    const T ws = w * sf, wd = w * dsf;
     const T u = ws * (sr * cs), v = ws * (sr * sn), p = fma(ws, A.psi_fac, -u);
     const T md[3] = {-n[0], -n[1], n[2]};  // m
     const T vm[3] = {v * md[0], v * md[1], v * md[2]};
@@ -504,8 +532,9 @@ __device__ __forceinline__ void plain_self_row(const PlainArgs<T> &A, int a, int
 // the FP32 accumulators.  Each component's P_g is summed over its blocks as integers (any
 // order gives the same bits, so warps add with shared-memory atomics) and converted once.
 // Both integers are scaled entry by entry with the power of two next to F: with one per row the
-// rounding grew with the range of F within a row, and dB/dr at lmax 6 (lmax 4) was 5.8e-15
-// (1.9e-15) off a 64-bit evaluation instead of 2.1e-15 (1.8e-15); plain FP64 sums 1.9e-15 (1.6e-15).
+// rounding grew with the range of F within a row (dB/dr at lmax 6 was 5.8e-15 off).  In an
+// emulation with 64-bit mantissas, stage by stage, this rounding alone puts dB/dr 2e-17 off; what is
+// left are the image's psi and Cayley-Klein parameters, 1.5e-15 at lmax 4 and 2.0e-15 at lmax 6.
 constexpr int DT = 192;    // threads: two CTAs per SM with 168 registers each
 constexpr int ND = 8;      // digits
 constexpr int VB = 61, ZB = 62;  // bits of V and W
@@ -982,10 +1011,10 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
             const pc<float> z = Zt[(size_t)ps.x * ZQ<float>], zq = Zt[(size_t)ps.z * ZQ<float>];
             pc<float> zn = Zt[(size_t)ps.y * ZQ<float>];
             if (ps.w & 1) zn.re = -zn.re;  // the mirror -conj(Z'[m-1]) past a middle row's centre
-            const float xr = f.z * zn.re, xi = f.z * zn.im, yr = f.w * zq.re, yi = f.w * zq.im;
+            const float yr = f.w * zq.re, yi = f.w * zq.im;
             // (re of W0..W3), (im of W0..W3)
-            W[2 * (e - w0)] = make_float4(f.x * z.re, f.y * z.im, xr - yr, xi + yi);
-            W[2 * (e - w0) + 1] = make_float4(f.x * z.im, -f.y * z.re, xi - yi, -(xr + yr));
+            W[2 * (e - w0)] = make_float4(f.x * z.re, f.y * z.im, fmaf(f.z, zn.re, -yr), fmaf(f.z, zn.im, yi));
+            W[2 * (e - w0) + 1] = make_float4(f.x * z.im, -f.y * z.re, fmaf(f.z, zn.im, -yi), -fmaf(f.z, zn.re, yr));
             vrow[e - w0] = (ps.w >> 1) * P;
         }
     };
@@ -1230,7 +1259,6 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
     A.wk = t->d_p_wk;
     A.wpos = t->d_p_wpos;
     A.wfac = t->d_p_wfac;
-    A.yscale = t->d_yscale;
     A.rc = (T)p->rcut;
     A.psi_fac = (T)(p->rfac0 * SO4_PI / p->rcut);
     fill_small_tables(t, A.st);
@@ -1256,7 +1284,7 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
             if ((rc = so4_set_smem((const void *)k_plain_u, smu))) return rc;
             k_plain_u<<<n, UT, smu, st>>>(A);
         } else {
-            rc = so4_utot32(t, p, n, w_nb, w_site + a0, img_ptr + a0, img_j, img_r, (float *)A.uh, st);
+            rc = so4_utot32_as(t, p, t->d_hmap_v, n, w_nb, w_site + a0, img_ptr + a0, img_j, img_r, (float *)A.uh, st);
             if (rc) return rc;
             k_plain_tile<<<nt, 256, 0, st>>>(A);
         }

@@ -89,6 +89,7 @@ void free_device(so4_tables *t) {
     cudaFree(t->d_yblk);
     cudaFree(t->d_hfull);
     cudaFree(t->d_hmap);
+    cudaFree(t->d_hmap_v);
     cudaFree(t->d_yscale);
     cudaFree(t->d_pz_unit);
     cudaFree(t->d_p_vent);
@@ -836,7 +837,7 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     // symmetry keep their form.  hmap: per half entry {slot | row << 8 | diagonal << 15,
     // bits of u_norm F, bits of u_norm, 0}; yscale: F, by which the window kernels scale Y so
     // that the reverse sweep contracts V with it.
-    std::vector<int4> hmap;
+    std::vector<int4> hmap, hmap_v;
     std::vector<float> yscale;
     for (int l = 0; l < ld; ++l) {
         const float un = (float)t->unorm_l[l];
@@ -848,11 +849,13 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
                 std::memcpy(&b_unf, &unf, sizeof b_unf);
                 std::memcpy(&b_un, &un, sizeof b_un);
                 hmap.push_back(make_int4((l * (l + 1) / 2 + ma) | (mb << 8) | ((ma == mb ? 1 : 0) << 15), b_unf, b_un, 0));
+                hmap_v.push_back(make_int4(hmap.back().x, b_un, b_un, 0));
                 yscale.push_back((float)F);
             }
     }
     if (!rc) rc = upload(&t->d_hfull, hfull);
     if (!rc) rc = upload(&t->d_hmap, hmap);
+    if (!rc) rc = upload(&t->d_hmap_v, hmap_v);
     if (!rc) rc = upload(&t->d_yscale, yscale);
     if (!rc) rc = upload(&t->d_bpos, bpos);
     if (!rc) rc = upload(&t->d_wunit_y, wunit_y);
