@@ -194,16 +194,17 @@ __global__ void __launch_bounds__(UT) k_plain_u(PlainArgs<double> A) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int e = tid + q * UT;
-                double pr[2] = {0.0, 0.0}, pi[2] = {0.0, 0.0};  // even and odd images of this part
-                if (e < nh)
+                if (e < nh) {
+                    double pr[2] = {0.0, 0.0}, pi[2] = {0.0, 0.0};  // even and odd images of this part
 #pragma unroll 2
                     for (int i = 0; i < nc; ++i) {
                         const pc<double> v = V[v_at(e, i)];
                         pr[i & 1] = fma(wsf[c0 + i], v.re, pr[i & 1]);
                         pi[i & 1] = fma(wsf[c0 + i], v.im, pi[i & 1]);
                     }
-                ar[q] += pr[0] + pr[1];
-                ai[q] += pi[0] + pi[1];
+                    ar[q] += pr[0] + pr[1];
+                    ai[q] += pi[0] + pi[1];
+                }
             }
             __syncthreads();
         }
