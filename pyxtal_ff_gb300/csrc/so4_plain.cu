@@ -404,12 +404,16 @@ __global__ void __launch_bounds__(256) k_plain_b(PlainArgs<T> A) {
     if (a < A.natoms) A.x[(size_t)a * A.n_b + k] = T(2) * s;
 }
 
-// 1 / v in FP32, from v = vh + vl: the quotient of vh corrected by its residual, within a few
-// thousandths of half an ulp.  (An FP64 division is some thirty instructions of a pipe with 1/64
-// of the FP32 rate, in the one warp that the CTA waits for.)
+// 1 / v in FP64, rounded to FP32: two Newton steps from FP32's quotient instead of an FP64 division
+// (some thirty instructions of a pipe with 1/64 of the FP32 rate, in the one warp that the CTA waits
+// for).  The first leaves 2^-46, the second FP64's own rounding.
 __device__ __forceinline__ float inv32(double v) {
-    const float vh = (float)v, vl = (float)(v - (double)vh), y = 1.f / vh;
-    return fmaf(fmaf(-vl, y, fmaf(-vh, y, 1.f)), y, y);
+    const float f = (float)v;
+    if (!(f > 1e-37f && f < 1e37f)) return (float)(1.0 / v);
+    double y = (double)(1.f / f);
+    y = fma(fma(-v, y, 1.0), y, y);
+    y = fma(fma(-v, y, 1.0), y, y);
+    return (float)y;
 }
 
 // ---------------------------------------------------------------- dB/dr
