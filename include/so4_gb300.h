@@ -248,8 +248,12 @@ int so4_status_read(const void *d_work, size_t work_bytes, void *stream, int *h_
  * number; SNAP: 1).  want_deriv / want_stress as the reference's flags; dxdr
  * and rdxdr may be NULL when not wanted.  Output element type is double
  * (precision 0) or float (precision 1).  Scratch: so4_plain_workspace_size()
- * bytes -- a status header, and at twol 12, where the FP64 path's Z does not fit in
- * shared memory, one global Z slot per CTA of the launch (min(natoms, 2 x SMs)). */
+ * bytes, a header and U_tot and Z of the centres, 32 to a tile (at lmax 4 a tile takes
+ * 1.3 MB in FP64, 0.7 MB in FP32), 768 MB at most: more centres are taken in passes.  With
+ * less the passes are shorter (the same results bit for bit); with less than a tile, NULL
+ * too, the call allocates as much in the stream's order (cudaMallocAsync) and frees it
+ * behind its kernels, but for precision 0 at twol 12, where it returns
+ * SO4_ERR_WORKSPACE. */
 size_t so4_plain_workspace_size(const so4_tables *t, int natoms);
 int so4_plain(const so4_tables *t, const so4_params *p, int precision, const so4_geom *d_geom,
               const int *d_atom_struct, int natoms, const double *d_pos, const double *d_w_nb,

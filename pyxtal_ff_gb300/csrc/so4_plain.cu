@@ -1211,17 +1211,35 @@ size_t plain_tile_bytes(const so4_tables *t) {
     if (sizeof(T) == 4) b += sizeof(float2) * 32 * (size_t)t->n_half;
     return b;
 }
+// centres of a pass in that many bytes (0: not one tile)
 template <typename T>
-int plain_pass(const so4_tables *t, int natoms) {
+int plain_pass(const so4_tables *t, int natoms, size_t bytes) {
     // equal passes of whole tiles
-    const size_t most = std::max<size_t>(1, PLAIN_BYTES / plain_tile_bytes<T>(t)), tiles = ((size_t)natoms + 31) / 32;
+    const size_t most = std::min(bytes, PLAIN_BYTES) / plain_tile_bytes<T>(t), tiles = ((size_t)natoms + 31) / 32;
+    if (most == 0) return 0;
     const size_t np = std::max<size_t>(1, (tiles + most - 1) / most);
     return (int)std::min<size_t>((size_t)natoms, 32 * ((tiles + np - 1) / np));
 }
 template <typename T>
 size_t plain_scratch(const so4_tables *t, int natoms) {
-    return plain_tile_bytes<T>(t) * (size_t)((plain_pass<T>(t, natoms) + 31) / 32);
+    return plain_tile_bytes<T>(t) * (size_t)((plain_pass<T>(t, natoms, PLAIN_BYTES) + 31) / 32);
 }
+
+// Scratch of the call's own, in the stream's order, for a caller who gave none.
+struct OwnScratch {
+    void *p = nullptr;
+    cudaStream_t st;
+    explicit OwnScratch(cudaStream_t s) : st(s) {}
+    ~OwnScratch() {
+        if (p) cudaFreeAsync(p, st);
+    }
+    int take(size_t bytes) {
+        if (cudaMallocAsync(&p, bytes, st) == cudaSuccess) return SO4_OK;
+        p = nullptr;
+        cudaGetLastError();
+        return SO4_ERR_WORKSPACE;
+    }
+};
 
 template <typename T>
 int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, const int *astruct, int natoms,
@@ -1272,10 +1290,20 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
     A.dxdr = (T *)dxdr;
     A.rdxdr = (T *)rdxdr;
     A.cw = t->p_cw;
-    const int pass = plain_pass<T>(t, natoms);
-    if (!work || work_bytes < SO4_WS_HEADER + plain_scratch<T>(t, natoms)) return SO4_ERR_WORKSPACE;
+    // As many centres a pass as the caller's scratch holds; without a tile's worth the call takes
+    // its own (but for FP64 at twol 12, which always asked for scratch).
+    OwnScratch own(st);
+    char *base = work ? (char *)work + SO4_WS_HEADER : nullptr;
+    int pass = plain_pass<T>(t, natoms, work && work_bytes > SO4_WS_HEADER ? work_bytes - SO4_WS_HEADER : 0);
+    if (pass == 0) {
+        if (sizeof(T) == 8 && t->twol == 12) return SO4_ERR_WORKSPACE;
+        const int rc = own.take(plain_scratch<T>(t, natoms));
+        if (rc) return rc;
+        base = (char *)own.p;
+        pass = plain_pass<T>(t, natoms, PLAIN_BYTES);
+    }
     const size_t tiles = (size_t)(pass + 31) / 32;
-    A.ut = (pc<T> *)((char *)work + SO4_WS_HEADER);
+    A.ut = (pc<T> *)base;
     A.zt = A.ut + tiles * 32 * t->n_u;
     A.zi = (longlong2 *)(A.zt + tiles * 32 * t->n_pz);
     A.uh = (float2 *)A.zi;
@@ -1293,7 +1321,6 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
             if (rc) return rc;
             k_plain_tile<<<nt, 256, 0, st>>>(A);
         }
-        // a tile's units over as many CTAs as it takes to give every SM several
         // A tile's Z units are spread over up to n_unit / 16 CTAs while the grid has fewer than eight
         // CTAs per SM: 64 centres (two tiles) at lmax 3 would otherwise run on two SMs.
         const int parts = std::max(1, std::min((A.n_unit + 15) / 16, 1216 / nt));
