@@ -173,7 +173,7 @@ class PyXtalFFCalculator:
         return energies[order], forces, stress[0] / EV_A3_TO_GPA * EV2GPA
 
     def _plain(self, atoms, ff):
-        if type(ff.model).calculate_properties is not NeuralNetworkPotential.calculate_properties:
+        if getattr(ff.model.calculate_properties, "__func__", None) is not NeuralNetworkPotential.calculate_properties:
             self.desp = compute_descriptor(ff._descriptors, atoms)
             return ff.model.calculate_properties(self.desp, bforce=True, bstress=True)
         # the same two calls with the descriptors left on the device between them

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 import torch
 
+from pyxtal_ff_gb300 import ase_calculator as A
 from pyxtal_ff_gb300 import calculator as C
 from pyxtal_ff_gb300 import structures as S
 from pyxtal_ff_gb300.ase_calculator import ForceField, PyXtalFFCalculator
@@ -97,6 +98,25 @@ def test_periodicity_or_networks_alone_are_a_change(monkeypatch):
     assert _Fake.made[0].log == ["compute"] * 3
     held = calc._last_key  # the objects, not their ids
     assert any(m is calc.parameters["ff"].model for m in held) and (calc.parameters["ff"].model.models["Si"],) in held
+
+
+@pytest.mark.parametrize("where", ["subclass", "instance"])
+def test_plain_route_asks_a_model_of_its_own(monkeypatch, where):
+    """A model whose calculate_properties is not NeuralNetworkPotential's, by its class or on the object
+    alone, gets the descriptors (numpy) and gives the results."""
+    class Mine(NeuralNetworkPotential):
+        def calculate_properties(self, descriptor, bforce=True, bstress=False):
+            return np.full(2, descriptor["x"]), np.ones((2, 3)), np.zeros(6)
+
+    base = _potential("cpu")
+    if where == "subclass":
+        model = Mine(base.models, base.drange, device="cpu")
+    else:
+        model = base
+        model.calculate_properties = lambda d, bforce=True, bstress=False: Mine.calculate_properties(model, d)
+    monkeypatch.setattr(A, "compute_descriptor", lambda function, atoms: {"x": 3.5})
+    calc, atoms = PyXtalFFCalculator(ff=ForceField(DESC, model)), S.Atoms([14] * 2, np.eye(3)[:2], 9 * np.eye(3))
+    assert calc.get_potential_energy(atoms) == 7.0 and np.array_equal(calc.get_forces(atoms), np.ones((2, 3)))
 
 
 @pytest.mark.gpu
