@@ -14,7 +14,8 @@ device.  The knobs:
   zw_atoms     atoms per CTA of the window Z pass: 32 (one per lane) or 64 (two per lane,
                up to twol 8)
   zw_threads   threads per CTA of the 64-atom window pass, 256 or 512
-  branches     parallel graph branches of the captured linear step, 1..4
+  branches     parallel graph branches of the captured linear step, 1..4 (0: by the number of
+               atoms, as an untuned calculator takes them)
   pdl          programmatic dependent launch between that step's kernels
 
 The search is a coordinate descent from the defaults: each knob in turn takes every
@@ -42,11 +43,12 @@ SPACE_ORDER = ("branches", "wkmax", "zw_atoms", "zw_threads", "rev_pair", "rev_t
 
 @dataclass(frozen=True)
 class Choice:
-    """One point of the search space (0 in a kernel field: the table builder's default)."""
+    """One point of the search space (0 in a kernel field: the table builder's default; 0 branches:
+    the captured step's own rule)."""
     wkmax: int = 5
     rev_threads: int = 0
     utot_warps: int = 4
-    branches: int = 2
+    branches: int = 0
     pdl: bool = False
     rev_pair: int = 0
     zw_atoms: int = 0
@@ -83,7 +85,7 @@ def search_space(twol, linear=True):
 
 
 def default_choice(twol, linear=True):
-    return Choice(wkmax=5, rev_threads=0, utot_warps=4, branches=2 if linear else 1, pdl=False)
+    return Choice(wkmax=5, rev_threads=0, utot_warps=4, branches=0 if linear else 1, pdl=False)
 
 
 def coordinate_descent(evaluate, start, space, rounds=3, min_gain=0.01):
@@ -212,7 +214,7 @@ class Validator:
         del d
 
     def check(self, branches, pdl):
-        step = self.calc.capture(self.batch, self.model, branches=branches, pdl=pdl)
+        step = self.calc.capture(self.batch, self.model, branches=branches or None, pdl=pdl)
         res = step()
         ef = float((res["forces"] - self.f_ref).abs().max())
         es = float((res["stress"] - self.s_ref).abs().max())
@@ -250,7 +252,7 @@ def autotune_step(calc, batch, model, *, steps=20, warmup=5, rounds=3, use_cache
                 log("autotune: %r rejected (force err %.3g, stress err %.3g)" % (c, ef, es))
             return None
         calc.prepare(batch)
-        step = calc.capture(batch, model, branches=c.branches, pdl=c.pdl)
+        step = calc.capture(batch, model, branches=c.branches or None, pdl=c.pdl)
         t = _median_ms(step, steps, warmup)
         del step
         if log:

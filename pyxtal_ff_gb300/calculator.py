@@ -119,7 +119,8 @@ class SO4Calculator:
         self.tuning = tuning
         with torch.cuda.device(self.device):
             self.tables = engine.tables(self.twol, self.normalize_U, None if tuning is None else tuning.kernel_tuning())
-        self.branches = 2 if tuning is None else int(tuning.branches)
+        # of a captured linear step; 0: by the number of atoms (capture)
+        self.branches = 0 if tuning is None else int(tuning.branches)
         self.pdl = False if tuning is None else bool(tuning.pdl)
         self._ws = None
 
@@ -146,11 +147,11 @@ class SO4Calculator:
     def capture(self, batch: Batch, model, headroom=1.25, branches=None, pdl=None, host_io=False):
         """The whole energy / forces / stress step of this batch layout as one CUDA graph
         (see CapturedStep); call the result with new positions.  branches / pdl default to
-        the calculator's tuning (untuned: 2 above TWO_BRANCH_ATOMS, else 1, and off); host_io: the
+        the calculator's tuning (0 branches or untuned: 2 above TWO_BRANCH_ATOMS, else 1; pdl off); host_io: the
         graph also copies the positions in from, and the results out to, pinned host buffers of
         the step."""
         if branches is None:
-            branches = self.branches if self.tuning is not None or batch.natoms > TWO_BRANCH_ATOMS else 1
+            branches = self.branches or (2 if batch.natoms > TWO_BRANCH_ATOMS else 1)
         return CapturedStep(self, batch, model, headroom=headroom, branches=branches,
                             pdl=self.pdl if pdl is None else pdl, host_io=host_io)
 
