@@ -97,8 +97,9 @@ int so4_tables_destroy(so4_tables *t);
  *               work lists are built for it (a smaller unit: more units, fewer
  *               registers per ring, other rounding of the Z sums);
  *   rev_threads threads per CTA of the one-lane-per-row-chain per-image pass, 128 or
- *               256 (default 256 up to twol 8, 128 above; only twol 6 and 8 have both, and
- *               up to twol 5 the pass takes 128);
+ *               256 (default 256 up to twol 8, 128 above; only twol 6 and 8 have both.  Up
+ *               to twol 5 the name of the one shape is 256, as it was when it had as many
+ *               threads; it has 128 now);
  *   utot_warps  warps (centres) per CTA of the U_tot pass, 2, 4 or 8 (default 4; only
  *               twol 6 and 8 have all three);
  *   rev_pair    layout of the per-image pass: 1 two lanes per image (its row chains

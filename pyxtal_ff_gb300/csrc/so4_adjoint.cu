@@ -1097,9 +1097,11 @@ int launch_deidrj_rev_nt(const DArgs &D, int64_t nimg, cudaStream_t st) {
 // registers: 38,912 atoms of lmax 2 124 -> 108 us, of lmax 2.5 140 -> 126, two of 256 before; 256 for
 // twol 6 to 8, 128 above; both for twol 6, 8).  pair: two lanes per image (k_deidrj_rev2, twol 6 and
 // 8) instead of one lane per row chain; sixteen warps per SM at twol 6, by four CTAs where there are
-// many images (64,000 atoms 240 -> 230 us, 38,912 145 -> 140), by two below (4,096 atoms 18.5 us, by
-// four 19.3; 9,728, with 272,084 images, 37.3 and 37.6); three CTAs of 128 threads at twol 8.
-constexpr int64_t REV2_MANY = 400000;
+// many images, by two below; three CTAs of 128 threads at twol 8.  The line lies where neither is
+// ahead: by two and by four CTAs 28.2 and 28.7 us at 115,000 images, 43.0 and 42.2 at 224,000, 51.7
+// and 50.8 at 298,000, 65.8 and 64.5 at 419,000, 75.2 and 73.0 at 492,000, 150 and 144 at 1,099,000 (one
+// call with its launch, lmax 3).
+constexpr int64_t REV2_MANY = 200000;
 template <int TWOL>
 int launch_deidrj_rev(const DArgs &D, int64_t nimg, int nt, int pair, cudaStream_t st) {
     if constexpr (TWOL == 6 || TWOL == 8) {
