@@ -386,12 +386,13 @@ __global__ void __launch_bounds__(256) k_scan_images(const so4_geom *geom, const
                 if (!(lo > 0.f && d2 < lo * lo)) {     // within the rounding band: decide in FP64
                     if (!exact_inside(g, pi, pos, j, o[0], o[1], o[2], rcut)) continue;
                 }
+                // an image that no key can hold is not counted either: k_sort reads a key per image
+                if (abs(o[0]) > OFF_MAX || abs(o[1]) > OFF_MAX || abs(o[2]) > OFF_MAX) {
+                    flag(w.status, SO4_ERR_OFFSET);
+                    flag(w.status, SO4_ERR_CAPACITY);
+                    continue;
+                }
                 if (MODE >= 1) {
-                    if (abs(o[0]) > OFF_MAX || abs(o[1]) > OFF_MAX || abs(o[2]) > OFF_MAX) {
-                        flag(w.status, SO4_ERR_OFFSET);
-                        flag(w.status, SO4_ERR_CAPACITY);
-                        continue;
-                    }
                     const unsigned long long key = ((unsigned long long)(unsigned)j << 30) |
                                                    ((unsigned long long)(o[0] + OFF_BIAS) << 20) |
                                                    ((unsigned long long)(o[1] + OFF_BIAS) << 10) |

@@ -95,9 +95,27 @@ def test_ase_calculator_outlives_an_overflow(cuda_device):
 
 
 @pytest.mark.gpu
-def test_offset_beyond_the_encodable_range_is_still_an_error(cuda_device):
-    at = S.diamond_si(2, 2, 2, sigma=0.05, rng=np.random.default_rng(92))
+@pytest.mark.parametrize("cells", [(2, 2, 2), (6, 6, 5)])  # four warps and one per centre
+def test_offset_beyond_the_encodable_range_is_still_an_error(cuda_device, cells):
+    """Images that no key can hold are left out of the counts as well as of the keys: a count without
+    its key would have the sort read what the workspace held before (here bytes 0x7f)."""
+    at = S.diamond_si(*cells, sigma=0.05, rng=np.random.default_rng(92))
+    batch = Batch([at])
+    lay = engine.layout(batch.cells, batch.pbc, batch.atom_ptr, RCUT)
+    near = engine.build_neighbors(at.positions, batch.cells, batch.pbc, batch.atom_ptr, RCUT)
     pos = at.positions.copy()
     pos[5, 0] += 600 * at.get_cell()[0, 0]
-    with pytest.raises(_lib.SO4Error):
-        engine.build_neighbors(pos, at.get_cell()[None], at.get_pbc()[None], [0, len(pos)], RCUT)
+    own = int(near.img_ptr[6] - near.img_ptr[5])
+    for slots in (0, 64):
+        bufs = engine.NeighborBuffers.allocate(lay, 2 * near.nimg, 2 * near.npair, "cuda", slot_cap=slots)
+        bufs.ws.fill_(0x7f)
+        engine.enqueue_neighbors(lay, torch.from_numpy(pos).cuda(), bufs)
+        M, _, bits = bufs.summary_dev().tolist()
+        torch.cuda.synchronize()
+        assert M == near.nimg - 2 * own  # its images, and itself as the others' image
+        assert bits & (1 << _lib.SO4_ERR_OFFSET) and bits & (1 << _lib.SO4_ERR_CAPACITY)
+        assert not bufs.img_ptr.any()  # emptied
+    with pytest.raises(_lib.SO4Error) as err:
+        engine.build_neighbors(pos, batch.cells, batch.pbc, batch.atom_ptr, RCUT)
+    assert err.value.code == _lib.SO4_ERR_CAPACITY
+    torch.cuda.synchronize()
