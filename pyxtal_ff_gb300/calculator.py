@@ -246,7 +246,8 @@ class CapturedStep:
     For any other model of (B, species) whose forward can be captured (no host
     synchronisation; a species_index() method, as the NN potential's networks have,
     supplies the atoms of each species once): the list, U_tot and B, the model and its
-    gradient dE/dB, Y, the per-image dE/dr and the gather, on one stream.  Either way the
+    gradient dE/dB, Y, the per-image dE/dr and the gather, in one branch (the reverse
+    images beside them on a stream of their own).  Either way the
     results equal those of SO4Calculator.compute bit for bit.
 
     The image / pair buffers have a fixed capacity (the counts of the structure at

@@ -635,8 +635,8 @@ __device__ __forceinline__ void zw2_unit_k(int k, const ZLArgs &A, const int4 un
     zw2_unit<MODE, K>(A, un, Ul, coef, ca, a, lane);
 }
 
-// k_zw32 with two atoms per lane: 64 atoms per CTA of NT threads, one CTA per SM (the
-// two-atom U tiles of twol 8 take 155 KB).  The same work lists, modes and outputs.
+// k_zw32 with two atoms per lane: 64 atoms per CTA of NT threads, NCTA CTAs per SM (one above twol 6,
+// where the two-atom U tiles take 155 KB at twol 8).  The same work lists, modes and outputs.
 // The first A.full groups of 64 atoms have a CTA each; the others are shared by clusters of
 // A.parts CTAs, CTA r taking units r, r + parts, .., and the slot sums follow a cluster barrier,
 // in CTA 0 (zw_split below).

@@ -42,7 +42,6 @@ __device__ __forceinline__ cx<T> cmul(cx<T> a, cx<T> b) {
 }
 template <typename T>
 __device__ __forceinline__ cx<T> cscale(cx<T> a, T s) { return mk<T>(a.re * s, a.im * s); }
-// acc += a * b
 // Re(conj(a) * b)
 template <typename T>
 __device__ __forceinline__ T redot(cx<T> a, cx<T> b) { return a.re * b.re + a.im * b.im; }
@@ -108,22 +107,22 @@ struct so4_tables {
     //   p_blk     per block {component, first Z value, entries, level}; p_fac its factor
     //             times u_norm
     //   p_zent    per Z value: block | 64 + exponent << 16
-    //   p_kblk_w  the components, longest first {up to three blocks, their number | k << 8}
+    //   p_kord    the components, longest first
     //   p_wpos, p_wfac  the Z values in that order, position q owning entries [p_wk[q],
     //             p_wk[q + 1]): what the FP32 kernel forms the generators' W of
     //   p_sent    section entries of all levels: ma | centre of a middle row << 8 | 2 + its exponent
     //             less the one of ma + 1 << 16 | and of ma - 1 << 20
-    int4 *d_pz_unit = nullptr, *d_p_vent = nullptr, *d_p_lam = nullptr, *d_p_blk = nullptr, *d_p_kblk_w = nullptr;
+    int4 *d_pz_unit = nullptr, *d_p_vent = nullptr, *d_p_lam = nullptr, *d_p_blk = nullptr;
     double *d_pz_ca = nullptr, *d_pz_cb = nullptr;
     float *d_pz_ca32 = nullptr, *d_pz_cb32 = nullptr;
     double *d_p_fac = nullptr;
     int *d_p_sent = nullptr;
     int *d_p_bblk = nullptr;  // n_b: the block a component's B contracts
-    int *d_p_zent = nullptr, *d_p_wk = nullptr;
+    int *d_p_zent = nullptr, *d_p_wk = nullptr, *d_p_kord = nullptr;
     int4 *d_p_wpos = nullptr;
     float4 *d_p_wfac = nullptr;
     std::vector<int> p_wk;
-    int n_pz_unit = 0, n_pblk = 0, n_pz = 0, p_cw = 0;
+    int n_pz_unit = 0, n_pz = 0, p_cw = 0;
     // B partial slots of the window kernels: one per (window unit, B block), component k
     // owning slots [bpos[k], bpos[k + 1]) in row order
     int *d_bpos = nullptr;  // nB + 1

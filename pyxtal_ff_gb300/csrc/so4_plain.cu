@@ -58,18 +58,18 @@ template <typename T>
 struct PlainArgs {
     so4_params prm;
     int a0, natoms;  // centres a0 .. natoms - 1
-    int n_u, n_half, n_z, n_b, n_blk, n_unit;
+    int n_u, n_half, n_z, n_b, n_unit;
     T rc, psi_fac;  // rcut and rfac0 pi / rcut
     int cw;  // k_plain_d64: 2^cw bounds the weights in W, times 4
     const so4_geom *geom;
     const int *astruct;
     const double *pos, *w_nb, *w_site, *img_r;
     const int32_t *img_ptr, *img_j, *pair_ptr, *pair_img, *nsite;
-    const int4 *unit, *vent, *lam, *blk, *kblk;
+    const int4 *unit, *vent, *lam, *blk;
     const int2 *hfull;
     const T *ca, *cb;
     const double *fac;
-    const int *sent, *bblk, *zent, *wk;
+    const int *sent, *bblk, *zent, *wk, *kord;
     const int4 *wpos;
     const float4 *wfac;
     SmallTables st;
@@ -1074,7 +1074,7 @@ __global__ void __launch_bounds__(ST, KS == 1 ? 3 : 2) k_plain_d32(PlainArgs<flo
                 if (lane == 0) pos = atomicAdd(&s_comp, 1);
                 pos = __shfl_sync(0xffffffffu, pos, 0);
                 if (pos >= k1) break;
-                const int e1 = __ldg(A.wk + pos + 1) - w0, kk = __ldg(&A.kblk[pos].w) >> 8;
+                const int e1 = __ldg(A.wk + pos + 1) - w0, kk = __ldg(A.kord + pos);
                 float2 p01[4], p23[4];  // (P0, P1), (P2, P3) of images il + 8 i
 #pragma unroll
                 for (int i = 0; i < 4; ++i) p01[i] = p23[i] = make_float2(0.f, 0.f);
@@ -1254,7 +1254,6 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
     A.n_half = t->n_half;
     A.n_z = t->n_pz;
     A.n_b = t->n_b;
-    A.n_blk = t->n_pblk;
     A.n_unit = t->n_pz_unit;
     A.geom = geom;
     A.astruct = astruct;
@@ -1271,7 +1270,7 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
     A.vent = t->d_p_vent;
     A.lam = t->d_p_lam;
     A.blk = t->d_p_blk;
-    A.kblk = t->d_p_kblk_w;
+    A.kord = t->d_p_kord;
     A.hfull = t->d_hfull;
     A.ca = (const T *)(sizeof(T) == 8 ? (const void *)t->d_pz_ca : (const void *)t->d_pz_ca32);
     A.cb = (const T *)(sizeof(T) == 8 ? (const void *)t->d_pz_cb : (const void *)t->d_pz_cb32);

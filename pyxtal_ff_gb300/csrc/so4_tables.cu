@@ -102,7 +102,7 @@ void free_device(so4_tables *t) {
     cudaFree(t->d_p_fac);
     cudaFree(t->d_p_sent);
     cudaFree(t->d_p_bblk);
-    cudaFree(t->d_p_kblk_w);
+    cudaFree(t->d_p_kord);
     cudaFree(t->d_p_zent);
     cudaFree(t->d_p_wpos);
     cudaFree(t->d_p_wfac);
@@ -399,7 +399,6 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
         }
     }
     p_zof.push_back(pz);
-    t->n_pblk = (int)p_blk.size();
     t->n_pz = pz;
     for (int k = 0; k < t->n_b; ++k)
         for (int bi = 0; bi < t->n_blk; ++bi)
@@ -410,9 +409,8 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     std::vector<int4> p_wpos;
     std::vector<float4> p_wfac;
     std::vector<int> p_wk(t->n_b + 1, 0);
-    // longest component first; position q holds component p_kblk_w[q].w >> 8
+    // longest component first; position q holds component kord[q]
     std::vector<int> kord(t->n_b), klen(t->n_b, 0);
-    std::vector<int4> p_kblk_w;
     for (int k = 0; k < t->n_b; ++k) {
         const int bs[3] = {p_kblk[k].x, p_kblk[k].y, p_kblk[k].z};
         kord[k] = k;
@@ -421,7 +419,6 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     std::stable_sort(kord.begin(), kord.end(), [&](int x, int y) { return klen[x] > klen[y]; });
     for (int q = 0; q < t->n_b; ++q) {
         const int k = kord[q];
-        p_kblk_w.push_back(make_int4(p_kblk[k].x, p_kblk[k].y, p_kblk[k].z, p_kblk[k].w | (k << 8)));
         const int bs[3] = {p_kblk[k].x, p_kblk[k].y, p_kblk[k].z};
         for (int i = 0; i < p_kblk[k].w; ++i) {
             const int4 b = p_blk[bs[i]];
@@ -881,7 +878,7 @@ extern "C" int so4_tables_create_tuned(int twol, int normalize_u, const so4_tuni
     if (!rc) rc = upload(&t->d_p_fac, p_fac);
     if (!rc) rc = upload(&t->d_p_sent, p_sent);
     if (!rc) rc = upload(&t->d_p_bblk, p_bblk);
-    if (!rc) rc = upload(&t->d_p_kblk_w, p_kblk_w);
+    if (!rc) rc = upload(&t->d_p_kord, kord);
     t->p_wk = p_wk;
     if (!rc) rc = upload(&t->d_p_zent, p_zent);
     if (!rc) rc = upload(&t->d_p_wpos, p_wpos);

@@ -106,8 +106,6 @@ class BispectrumBase:
         caller reduces it after calculate() (pyxtal_ff/utilities/__init__.py:226-233):
         one (len(x), nB, 6) Voigt row block per centre, summed on the GPU, so the
         per-pair array never leaves the device."""
-        from .. import engine
-
         res, _ = self._device(atoms, atom_ids, stress_per_atom)
         self._to_host(res)
         self.clear_memory()
