@@ -251,8 +251,8 @@ int so4_status_read(const void *d_work, size_t work_bytes, void *stream, int *h_
  * (precision 0) or float (precision 1).  Scratch: so4_plain_workspace_size()
  * bytes, a header and U_tot and Z of the centres, 32 to a tile (at lmax 4 a tile takes
  * 1.3 MB in FP64, 0.7 MB in FP32), 768 MB at most: more centres are taken in passes.  With
- * less the passes are shorter (the same results bit for bit); with less than a tile, NULL
- * too, the call allocates as much in the stream's order (cudaMallocAsync) and frees it
+ * less, or where d_work is not 32-byte aligned, the passes are shorter (the same results bit for bit);
+ * with less than a tile, NULL too, the call allocates as much in the stream's order (cudaMallocAsync) and frees it
  * behind its kernels, but for precision 0 at twol 12, where it returns
  * SO4_ERR_WORKSPACE. */
 size_t so4_plain_workspace_size(const so4_tables *t, int natoms);

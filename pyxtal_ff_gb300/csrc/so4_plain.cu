@@ -41,6 +41,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 
 #include <cuda_fp16.h>
 
@@ -1290,10 +1291,12 @@ int run_plain(const so4_tables *t, const so4_params *p, const so4_geom *geom, co
     A.rdxdr = (T *)rdxdr;
     A.cw = t->p_cw;
     // As many centres a pass as the caller's scratch holds; without a tile's worth the call takes
-    // its own (but for FP64 at twol 12, which always asked for scratch).
+    // its own (but for FP64 at twol 12, which always asked for scratch).  The tiles start where 16-byte
+    // words can be read, whatever the caller's alignment.
     OwnScratch own(st);
-    char *base = work ? (char *)work + SO4_WS_HEADER : nullptr;
-    int pass = plain_pass<T>(t, natoms, work && work_bytes > SO4_WS_HEADER ? work_bytes - SO4_WS_HEADER : 0);
+    const size_t skip = SO4_WS_HEADER + (size_t)(-(uintptr_t)work & 31);
+    char *base = work ? (char *)work + skip : nullptr;
+    int pass = plain_pass<T>(t, natoms, work && work_bytes > skip ? work_bytes - skip : 0);
     if (pass == 0) {
         if (sizeof(T) == 8 && t->twol == 12) return SO4_ERR_WORKSPACE;
         const int rc = own.take(plain_scratch<T>(t, natoms));

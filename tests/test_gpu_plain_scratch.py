@@ -88,3 +88,21 @@ def test_without_scratch_under_capture(cuda_device):
             t.fill_(0)
         graph.replay()
         assert all(torch.equal(a, b) for a, b in zip(out, ref))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("twol", [4, 11])
+def test_scratch_at_any_address(cuda_device, twol, precision):
+    """A caller may carve the scratch out of a block of its own: below twol 12 and in FP32 the call
+    never asked for an alignment."""
+    call = _Call(twol, precision)
+    full = engine.lib().so4_plain_workspace_size(call.tab.handle, NATOMS)
+    block = torch.empty(full + 64, dtype=torch.uint8, device="cuda")
+    assert block.data_ptr() % 32 == 0
+    _, ref = call(block, full)
+    for at in (4, 8, 16, 31):
+        for size in (full, HEADER + _tile_bytes(twol, precision)):
+            block.fill_(0x5a)
+            rc, out = call(block[at:], size)
+            assert rc == 0 and all(torch.equal(a, b) for a, b in zip(out, ref)), (at, size)
+            assert bool((block[:at] == 0x5a).all()) and bool((block[at + size:] == 0x5a).all())
