@@ -31,9 +31,9 @@
 //
 // Measured on a GB300 (one pass with the neighbour list; before: one CTA per centre for
 // everything, dU by recursion, every lane of a warp computing the image's set-up): FP64, 32,000
-// Si atoms, 0.93 M images, lmax 4: 142.3 -> 26.1 ms (k_plain_d64 14.3, k_plain_z 7.9, k_plain_u
-// 3.2); FP32, 16,232 atoms in 256 structures, lmax 3: 2.92 -> 1.14 ms.  k_plain_z is bound by the
-// FP64 pipe (91 % busy), k_plain_u too (80 %); k_plain_d64 by latency at twelve warps per SM: of
+// Si atoms, 0.93 M images, lmax 4: 142.3 -> 25.7 ms (k_plain_d64 13.8, k_plain_z 7.9, k_plain_u
+// 3.3); FP32, 16,232 atoms in 256 structures, lmax 3: 2.92 -> 1.04 ms.  k_plain_z is bound by the
+// FP64 pipe (95 % busy), k_plain_u too (91 %); k_plain_d64 by latency at twelve warps per SM: of
 // a CTA's 263,000 cycles the digit products take 115,000 (integer and shared-memory work around
 // the matrix instructions), V 48,000, the rows 46,000 (FP64), the set-up beside the rounding of
 // Z' 25,000.
